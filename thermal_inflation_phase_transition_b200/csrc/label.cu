@@ -12,13 +12,19 @@
 //
 // Method (union-find with atomic-min hooking, Playne & Hawick, "A new
 // algorithm for parallel connected-component labelling on GPUs", IEEE TPDS
-// 2018): every masked site starts as its own root; each site unites with its
-// +x, +y, +z masked neighbours by hooking the larger root under the smaller
-// one with atomicMin, so a component's root ends as its smallest linear
-// index; a pass of path compression leaves every site pointing at its root;
-// roots are ranked in index order (per-chunk counts, one scan, per-chunk
-// ballots) and the ranks are gathered back to the sites.  Every chase loop is
+// 2018): two masked neighbours unite by hooking the larger root under the
+// smaller one with atomicMin, so a component's root ends as its smallest linear
+// index.  Tiles of 2048 sites are labelled in shared memory first, where a run of
+// masked sites along a row is one entry (its start, from the row's ballot) and
+// two rows unite once per overlapping pair of runs; then the pairs across tile
+// faces unite in global memory; roots are ranked in index order (per-chunk
+// ranks, one scan) and every site gathers its root's rank.  Every chase loop is
 // bounded; an exhausted bound sets the status word to TIPT_ERR_TIMEOUT.
+//
+// Bound: the latency of the chases and the passes over the labels (20 bytes a
+// site, L2 resident up to about 2e7 sites).  250x243x237 float32, one label call:
+// 819 us with a union per site and direction in global memory and seven passes,
+// 238 us here (tiles 88, faces 54, ranks 12, gather 36 of it).
 #include "tipt_device.cuh"
 #include "tipt_internal.h"
 
@@ -48,11 +54,12 @@ __device__ __forceinline__ double field_val(const void* f, int64_t s, int64_t N)
     }
 }
 
+// |field| > thr.  float32: thrf is the largest float <= thr, which no float
+// separates from thr, so the comparison needs no conversion.
 template <int S>
-__global__ void label_init_kernel(const void* f, double thr, int32_t* L, int64_t N) {
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N;
-         s += (int64_t)gridDim.x * blockDim.x)
-        L[s] = field_abs<S>(f, s, N) > thr ? (int32_t)s : -1;
+__device__ __forceinline__ bool above(const void* f, int64_t s, int64_t N, double thr, float thrf) {
+    if constexpr (S == TIPT_F32) return fabsf(__ldg(static_cast<const float*>(f) + s)) > thrf;
+    else return field_abs<S>(f, s, N) > thr;
 }
 
 __device__ __forceinline__ int32_t find_root(const int32_t* L, int32_t x, bool& ok) {
@@ -65,10 +72,27 @@ __device__ __forceinline__ int32_t find_root(const int32_t* L, int32_t x, bool& 
     return x;
 }
 
+// find_root that halves the path behind it (each site visited is linked to its
+// grandparent).  Only non-roots are written, with an ancestor of theirs; a hook
+// that such a store overwrites is not lost, because unite() goes on with the value
+// that its atomicMin returned unless it hooked a root.
+__device__ __forceinline__ int32_t find_halving(int32_t* L, int32_t x, bool& ok) {
+    for (int it = 0; it < kChase; ++it) {
+        const int32_t y = L[x];
+        if (y == x) return x;
+        const int32_t z = L[y];
+        if (z == y) return y;
+        L[x] = z;
+        x = z;
+    }
+    ok = false;
+    return x;
+}
+
 __device__ __forceinline__ void unite(int32_t* L, int32_t a, int32_t b, bool& ok) {
     for (int it = 0; it < kChase && ok; ++it) {
-        a = find_root(L, a, ok);
-        b = find_root(L, b, ok);
+        a = find_halving(L, a, ok);
+        b = find_halving(L, b, ok);
         if (a == b) return;
         if (a < b) {
             const int32_t old = atomicMin(&L[b], a);
@@ -83,71 +107,220 @@ __device__ __forceinline__ void unite(int32_t* L, int32_t a, int32_t b, bool& ok
     ok = false;
 }
 
-__global__ void label_merge_kernel(int32_t* L, int n0, int n1, int n2, int periodic) {
-    const int64_t n12 = (int64_t)n1 * n2, N = (int64_t)n0 * n12;
-    bool ok = true;
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        if (L[s] < 0) continue;
-        const int k = (int)(s % n2);
-        const int64_t r = s / n2;
-        const int j = (int)(r % n1);
-        const int i = (int)(r / n1);
-        int64_t nb[3] = {-1, -1, -1};
-        if (i + 1 < n0) nb[0] = s + n12;
-        else if (periodic && n0 > 1) nb[0] = s - (int64_t)(n0 - 1) * n12;
-        if (j + 1 < n1) nb[1] = s + n2;
-        else if (periodic && n1 > 1) nb[1] = s - (int64_t)(n1 - 1) * n2;
-        if (k + 1 < n2) nb[2] = s + 1;
-        else if (periodic && n2 > 1) nb[2] = s - (n2 - 1);
+// Masks of up to 32 sites: the first column of the run that holds column q, and
+// the run that starts at column q.
+__device__ __forceinline__ int run_start(uint32_t m, int q) {
+    const uint32_t gap = ~m & ((1u << q) - 1u);
+    return gap ? 32 - __clz((int)gap) : 0;
+}
+__device__ __forceinline__ uint32_t run_mask(uint32_t m, int q) {
+    const uint32_t end = ~(m >> q);                 // bit 0 is clear
+    const int len = end ? __ffs((int)end) - 1 : 32;
+    return (len < 32 ? (1u << len) - 1u : 0xffffffffu) << q;
+}
+
+// Labels of one tile of TI x TJ rows of TK sites: L[s] = linear index of the
+// smallest site of s's component within the tile (-1 where not masked).  Warps read
+// rows (8 passes of 32 / TK rows) into masks; then one thread per row walks its
+// runs, so that a warp works on 32 rows at once (a lane per site spent 2.5 times the
+// instructions: most lanes idle in every union); then warps write rows.
+template <int S, int TI, int TJ, int TK>
+__global__ void __launch_bounds__(256) label_tile_kernel(const void* f, double thr, float thrf,
+                                                         int32_t* L, int n0, int n1, int n2) {
+    constexpr int RPW = 32 / TK;  // rows per warp and pass
+    constexpr int RS = TK + 1;    // entries per row, odd: rows in different banks
+    static_assert(TI * TJ * TK == 2048 && 32 % TK == 0, "eight warps of eight passes");
+    __shared__ int32_t s_l[TI * TJ * RS];  // union-find over the runs, at their first column
+    __shared__ uint32_t s_m[TI * TJ];      // mask of each row
+    const int ntk = (n2 + TK - 1) / TK, ntj = (n1 + TJ - 1) / TJ;
+    const int tk = blockIdx.x % ntk, tr = blockIdx.x / ntk;
+    const int ti = tr / ntj, tj = tr - ti * ntj;
+    const int lane = threadIdx.x & 31, sub = lane / TK, c = lane % TK;
+    const int row0 = (threadIdx.x >> 5) * 8 * RPW + sub, k = tk * TK + c;
+    const int64_t N = (int64_t)n0 * n1 * n2;
+    bool on[8];
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-            if (nb[d] >= 0 && L[nb[d]] >= 0) unite(L, (int32_t)s, (int32_t)nb[d], ok);
+    for (int it = 0; it < 8; ++it) {
+        const int row = row0 + it * RPW, i = ti * TI + row / TJ, j = tj * TJ + row % TJ;
+        on[it] = i < n0 && j < n1 && k < n2 && above<S>(f, (i * n1 + j) * n2 + k, N, thr, thrf);
+    }
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+        uint32_t m = __ballot_sync(0xffffffffu, on[it]) >> (sub * TK);
+        if constexpr (TK < 32) m &= (1u << TK) - 1u;
+        if (c == 0) s_m[row0 + it * RPW] = m;
+    }
+    __syncthreads();
+    const int row = threadIdx.x;
+    const bool walks = row < TI * TJ;
+    const uint32_t m = walks ? s_m[row] : 0u;
+    const uint32_t mj = walks && row % TJ > 0 ? s_m[row - 1] : 0u;   // the row above (j - 1)
+    const uint32_t mi = walks && row >= TJ ? s_m[row - TJ] : 0u;     // the row behind (i - 1)
+    bool ok = true;
+    // a run starts under the first run of the row above that it touches, or else of
+    // the row behind: no union needed for that one
+    for (uint32_t rest = m; rest;) {
+        const int q = __ffs((int)rest) - 1;
+        const uint32_t run = run_mask(rest, q);
+        rest &= ~run;
+        int parent = row * RS + q;
+        if (run & mj) parent = (row - 1) * RS + run_start(mj, __ffs((int)(run & mj)) - 1);
+        else if (run & mi) parent = (row - TJ) * RS + run_start(mi, __ffs((int)(run & mi)) - 1);
+        s_l[row * RS + q] = parent;
+    }
+    __syncthreads();
+    // the other overlaps unite; one with the row behind adds nothing where the rows
+    // above both of them touch it in one column
+    const uint32_t both = mj && mi ? m & mj & mi & s_m[row - TJ - 1] : 0u;
+    for (uint32_t rest = m; rest;) {
+        const int q = __ffs((int)rest) - 1;
+        const uint32_t run = run_mask(rest, q);
+        rest &= ~run;
+        uint32_t o = run & mj;
+        if (o) o &= ~run_mask(o, __ffs((int)o) - 1);
+        for (; o;) {
+            const int x = __ffs((int)o) - 1;
+            o &= ~run_mask(o, x);
+            unite(s_l, row * RS + q, (row - 1) * RS + run_start(mj, x), ok);
+        }
+        o = run & mi;
+        if (o && !(run & mj)) o &= ~run_mask(o, __ffs((int)o) - 1);
+        for (; o;) {
+            const int x = __ffs((int)o) - 1;
+            const uint32_t ov = run_mask(o, x);
+            o &= ~ov;
+            if (!(ov & both)) unite(s_l, row * RS + q, (row - TJ) * RS + run_start(mi, x), ok);
+        }
+    }
+    __syncthreads();
+    for (uint32_t rest = m; rest;) {
+        const int q = __ffs((int)rest) - 1;
+        rest &= ~run_mask(rest, q);
+        s_l[row * RS + q] = find_root(s_l, row * RS + q, ok);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+        const int row = row0 + it * RPW, i = ti * TI + row / TJ, j = tj * TJ + row % TJ;
+        if (i >= n0 || j >= n1 || k >= n2) continue;
+        int32_t l = -1;
+        if (on[it]) {
+            const int r = s_l[row * RS + run_start(s_m[row], c)], rr = r / RS;
+            l = ((ti * TI + rr / TJ) * n1 + tj * TJ + rr % TJ) * n2 + tk * TK + r % RS;
+        }
+        L[(i * n1 + j) * n2 + k] = l;
     }
     if (!ok) atomicExch(&g_label_status, (int)TIPT_ERR_TIMEOUT);
 }
 
-__global__ void label_compress_kernel(int32_t* L, int64_t N) {
+// Unions across the tile faces normal to blockIdx.y (0: i, 1: j, 2: k) and, on a
+// periodic lattice, across its boundary.  Consecutive threads take neighbouring
+// pairs, and a pair beside another masked pair of the same two tiles adds nothing.
+__global__ void __launch_bounds__(256) label_faces_kernel(int32_t* L, int n0, int n1, int n2,
+                                                          int TI, int TJ, int TK, int periodic) {
+    const int d = blockIdx.y;
+    const int n[3] = {n0, n1, n2}, t[3] = {TI, TJ, TK};
+    const int st[3] = {n1 * n2, n2, 1};
+    // direction d, the outer and the inner (consecutive threads) of the other two
+    const int in = d == 2 ? 1 : 2, ou = d == 0 ? 1 : 0;
+    const unsigned inner = (unsigned)(n1 * n2), nf = (unsigned)((n[d] - 1) / t[d]);
+    const unsigned faces = nf + (periodic && n[d] > 1 ? 1u : 0u);
+    const unsigned per = d == 0 ? inner : (unsigned)n[ou] * (unsigned)n[in];
+    const unsigned total = faces * per;   // <= N + per < 2^32 (N < 2^31 sites)
+    const int lane = threadIdx.x & 31;
     bool ok = true;
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N;
-         s += (int64_t)gridDim.x * blockDim.x)
-        if (L[s] >= 0) L[s] = find_root(L, L[s], ok);
+    for (unsigned q0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); q0 < total;
+         q0 += gridDim.x * blockDim.x) {
+        const unsigned q = q0 + lane;
+        bool pair = false;
+        int32_t s = 0, o = 0;
+        int a = 0, b = 0;
+        if (q < total) {
+            const unsigned face = q / per, rem = q - face * per;
+            b = (int)(rem / (unsigned)n[in]);
+            a = (int)(rem - (unsigned)b * (unsigned)n[in]);
+            const int x = face < nf ? (int)(face + 1) * t[d] : 0;
+            s = x * st[d] + b * st[ou] + a * st[in];
+            o = x > 0 ? s - st[d] : s + (n[d] - 1) * st[d];
+            pair = L[s] >= 0 && L[o] >= 0;
+        }
+        const bool before = __shfl_up_sync(0xffffffffu, pair, 1);
+        // the pair before it, in either direction along the face, joins the same runs
+        if (pair && !(before && lane > 0 && a % t[in] != 0) &&
+            !(b % t[ou] != 0 && L[s - st[ou]] >= 0 && L[o - st[ou]] >= 0))
+            unite(L, s, o, ok);
+    }
     if (!ok) atomicExch(&g_label_status, (int)TIPT_ERR_TIMEOUT);
 }
 
-// roots per chunk (a root is a masked site that is its own label)
-__global__ void label_count_kernel(const int32_t* L, int64_t N, int32_t* chunk_roots) {
-    __shared__ int32_t s_cnt;
-    if (threadIdx.x == 0) s_cnt = 0;
+// Ranks of the roots (masked sites that are their own label) within their chunk
+// of kChunk sites, in index order: R[root] = rank, and the chunk's number of
+// roots.  A warp takes kChunk / 8 consecutive sites, 32 at a time; its lanes keep
+// their flags in the bits of a word.
+__global__ void __launch_bounds__(256) label_rank_kernel(const int32_t* L, int64_t N, int32_t* R,
+                                                         int32_t* chunk_roots) {
+    static_assert(kChunk == 8 * 32 * 32, "a flag word per lane");
+    __shared__ int32_t s_warp[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t b0 = (int64_t)blockIdx.x * kChunk + warp * (kChunk / 8) + lane;
+    uint32_t flags = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        int32_t l[16];  // sixteen loads in flight
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int64_t s = b0 + (h * 16 + q) * 32;
+            l[q] = s < N ? __ldg(L + s) : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+            flags |= (l[q] == (int32_t)(b0 + (h * 16 + q) * 32) ? 1u : 0u) << (h * 16 + q);
+    }
+    const int32_t cnt = (int32_t)__reduce_add_sync(0xffffffffu, __popc(flags));
+    if (lane == 0) s_warp[warp] = cnt;
     __syncthreads();
-    const int64_t b0 = (int64_t)blockIdx.x * kChunk;
-    int32_t c = 0;
-    for (int64_t s = b0 + threadIdx.x; s < b0 + kChunk && s < N; s += blockDim.x) c += L[s] == (int32_t)s;
-    atomicAdd(&s_cnt, c);
-    __syncthreads();
-    if (threadIdx.x == 0) chunk_roots[blockIdx.x] = s_cnt;
+    int32_t base = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w < warp) base += s_warp[w];
+        total += s_warp[w];
+    }
+    if (threadIdx.x == 0) chunk_roots[blockIdx.x] = total;
+    // the passes with a root in them
+    uint32_t any = __reduce_or_sync(0xffffffffu, flags);
+    while (any) {
+        const int it = __ffs(any) - 1;
+        any &= any - 1;
+        const unsigned m = __ballot_sync(0xffffffffu, flags >> it & 1u);
+        if (flags >> it & 1u) R[b0 + it * 32] = base + __popc(m & ((1u << lane) - 1u));
+        base += __popc(m);
+    }
 }
 
 // exclusive scan of the chunk counts (one block) and the total
-__global__ void label_scan_kernel(int32_t* chunk_roots, int n_chunks, int32_t* n_labels) {
-    __shared__ int32_t s_part[1024];
+__global__ void __launch_bounds__(1024) label_scan_kernel(int32_t* chunk_roots, int n_chunks,
+                                                          int32_t* n_labels) {
+    __shared__ int32_t s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = (n_chunks + blockDim.x - 1) / blockDim.x;
     const int b = threadIdx.x * per;
     int32_t sum = 0;
     for (int q = b; q < b + per && q < n_chunks; ++q) sum += chunk_roots[q];
-    s_part[threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int32_t run = 0;
-        for (int t = 0; t < (int)blockDim.x; ++t) {
-            const int32_t v = s_part[t];
-            s_part[t] = run;
-            run += v;
+    const auto warp_scan = [&](int32_t v) {   // inclusive
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
         }
-        *n_labels = run;
-    }
+        return v;
+    };
+    const int32_t inc = warp_scan(sum);
+    if (lane == 31) s_warp[warp] = inc;
     __syncthreads();
-    int32_t run = s_part[threadIdx.x];
+    if (warp == 0) s_warp[lane] = warp_scan(s_warp[lane]);
+    __syncthreads();
+    int32_t run = inc - sum + (warp ? s_warp[warp - 1] : 0);
+    if (threadIdx.x == blockDim.x - 1) *n_labels = run + sum;
     for (int q = b; q < b + per && q < n_chunks; ++q) {
         const int32_t v = chunk_roots[q];
         chunk_roots[q] = run;
@@ -155,41 +328,29 @@ __global__ void label_scan_kernel(int32_t* chunk_roots, int n_chunks, int32_t* n
     }
 }
 
-// rank the roots of a chunk in index order: R[root] = label (1-based)
-__global__ void label_rank_kernel(const int32_t* L, int64_t N, const int32_t* chunk_base,
-                                  int32_t* R) {
-    __shared__ int32_t s_warp[33];
-    const int64_t b0 = (int64_t)blockIdx.x * kChunk;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int32_t base = chunk_base[blockIdx.x];
-    for (int64_t off = 0; off < kChunk; off += blockDim.x) {
-        const int64_t s = b0 + off + threadIdx.x;
-        const bool root = s < N && L[s] == (int32_t)s;
-        const unsigned m = __ballot_sync(0xffffffffu, root);
-        if (lane == 0) s_warp[warp] = __popc(m);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int32_t run = 0;
-            for (int w = 0; w < nw; ++w) {
-                const int32_t v = s_warp[w];
-                s_warp[w] = run;
-                run += v;
-            }
-            s_warp[32] = run;
-        }
-        __syncthreads();
-        if (root) R[s] = base + s_warp[warp] + __popc(m & ((1u << lane) - 1u)) + 1;
-        base += s_warp[32];
-        __syncthreads();
+// label (1-based) of every site: its root's rank in the chunk plus the chunk's base
+__global__ void __launch_bounds__(256) label_gather_kernel(const int32_t* L, const int32_t* R,
+                                                           const int32_t* chunk_base, int32_t* out,
+                                                           int64_t N) {
+    bool ok = true;
+    // four sites a thread, so that four chases are in flight
+    for (int64_t s = (int64_t)blockIdx.x * 1024 + threadIdx.x; s < N; s += (int64_t)gridDim.x * 1024) {
+        int32_t l[4], r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) l[q] = s + 256 * q < N ? __ldg(L + s + 256 * q) : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[q] = l[q] >= 0 ? __ldg(L + l[q]) : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (r[q] != l[q]) r[q] = find_root(L, r[q], ok);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            l[q] = r[q] >= 0 ? __ldg(chunk_base + r[q] / kChunk) + __ldg(R + r[q]) + 1 : 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (s + 256 * q < N) out[s + 256 * q] = l[q];
     }
-}
-
-__global__ void label_gather_kernel(const int32_t* L, const int32_t* R, int32_t* out, int64_t N) {
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t l = L[s];
-        out[s] = l < 0 ? 0 : R[l];
-    }
+    if (!ok) atomicExch(&g_label_status, (int)TIPT_ERR_TIMEOUT);
 }
 
 // per-label statistics (index 0 = background, left at zero)
@@ -241,6 +402,33 @@ static int grid_for(int64_t N) {
     return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
 
+// Tile labels, then the unions across tile faces.  Tiles: 8 x 8 rows of 32 sites,
+// 8 x 32 rows of 8 for short rows (fewer than 20 sites would leave lanes of the
+// 32-site rows idle), 64 rows of 32 of a single plane.
+template <int S, int TI, int TJ, int TK>
+static void launch_tiles_as(const void* field, double thr, int32_t* L, int n0, int n1, int n2,
+                            bool periodic, cudaStream_t st) {
+    float thrf = (float)thr;
+    if ((double)thrf > thr) thrf = nextafterf(thrf, -INFINITY);
+    const int64_t tiles = (int64_t)((n0 + TI - 1) / TI) * ((n1 + TJ - 1) / TJ) * ((n2 + TK - 1) / TK);
+    label_tile_kernel<S, TI, TJ, TK><<<(unsigned)tiles, 256, 0, st>>>(field, thr, thrf, L, n0, n1, n2);
+    // the direction with the most face pairs sets the grid
+    const int64_t N = (int64_t)n0 * n1 * n2;
+    const int64_t pi = ((n0 - 1) / TI + 1) * (N / n0), pj = ((n1 - 1) / TJ + 1) * (N / n1),
+                  pk = ((n2 - 1) / TK + 1) * (N / n2);
+    const int64_t most = pi > pj ? (pi > pk ? pi : pk) : (pj > pk ? pj : pk);
+    label_faces_kernel<<<dim3((unsigned)grid_for(most), 3), 256, 0, st>>>(L, n0, n1, n2, TI, TJ, TK,
+                                                                          periodic ? 1 : 0);
+}
+
+template <int S>
+static void launch_tiles(const void* field, double thr, int32_t* L, int n0, int n1, int n2,
+                         bool periodic, cudaStream_t st) {
+    if (n0 == 1) launch_tiles_as<S, 1, 64, 32>(field, thr, L, n0, n1, n2, periodic, st);
+    else if (n2 < 20) launch_tiles_as<S, 8, 32, 8>(field, thr, L, n0, n1, n2, periodic, st);
+    else launch_tiles_as<S, 8, 8, 32>(field, thr, L, n0, n1, n2, periodic, st);
+}
+
 int64_t label_workspace_bytes(int64_t N) {
     const int64_t chunks = (N + kChunk - 1) / kChunk;
     return 4 * (2 * N + chunks + 64);
@@ -285,18 +473,22 @@ extern "C" int tipt_label_components(int storage, const void* field, double thre
     int32_t* R = L + N;
     int32_t* cr = R + N;
     cudaStream_t st = (cudaStream_t)stream;
-    const int g = grid_for(N);
-    switch (storage) {
-        case TIPT_F64: label_init_kernel<TIPT_F64><<<g, 256, 0, st>>>(field, threshold, L, N); break;
-        case TIPT_F32: label_init_kernel<TIPT_F32><<<g, 256, 0, st>>>(field, threshold, L, N); break;
-        default: label_init_kernel<TIPT_F32C><<<g, 256, 0, st>>>(field, threshold, L, N); break;
+    // (nx, ny, 1) has the components, indices and neighbours of (1, nx, ny), and
+    // (nx, 1, 1) those of (1, 1, nx)
+    int n0 = (int)nx, n1 = (int)ny, n2 = (int)nz;
+    if (n2 == 1) {
+        n2 = n1 > 1 ? n1 : n0;
+        n1 = n1 > 1 ? n0 : 1;
+        n0 = 1;
     }
-    label_merge_kernel<<<g, 256, 0, st>>>(L, (int)nx, (int)ny, (int)nz, periodic ? 1 : 0);
-    label_compress_kernel<<<g, 256, 0, st>>>(L, N);
-    label_count_kernel<<<(unsigned)chunks, 256, 0, st>>>(L, N, cr);
+    switch (storage) {
+        case TIPT_F64: launch_tiles<TIPT_F64>(field, threshold, L, n0, n1, n2, periodic != 0, st); break;
+        case TIPT_F32: launch_tiles<TIPT_F32>(field, threshold, L, n0, n1, n2, periodic != 0, st); break;
+        default: launch_tiles<TIPT_F32C>(field, threshold, L, n0, n1, n2, periodic != 0, st); break;
+    }
+    label_rank_kernel<<<(unsigned)chunks, 256, 0, st>>>(L, N, R, cr);
     label_scan_kernel<<<1, 1024, 0, st>>>(cr, (int)chunks, n_labels);
-    label_rank_kernel<<<(unsigned)chunks, 256, 0, st>>>(L, N, cr, R);
-    label_gather_kernel<<<g, 256, 0, st>>>(L, R, labels, N);
+    label_gather_kernel<<<grid_for((N + 3) / 4), 256, 0, st>>>(L, R, cr, labels, N);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "labelling launch");
 }
