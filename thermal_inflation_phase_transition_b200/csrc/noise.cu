@@ -1,5 +1,7 @@
 // Counter-based noise kernels: the hash pairs themselves (parity checks) and
 // the noise-field fill that replaces the MT19937 generate_noise_field.
+#include <type_traits>
+
 #include "tipt_device.cuh"
 #include "tipt_internal.h"
 
@@ -13,20 +15,25 @@ __global__ void hash_pairs_kernel(const uint64_t* __restrict__ keys, int64_t n, 
         hash_pair(keys[q], a, b);
         if (u1) u1[q] = a;
         if (u2) u2[q] = b;
-        if (z) z[q] = bm_radius(a) * cos(kTwoPiLit * b);
+        if (z) z[q] = gauss_cos(keys[q]);
     }
 }
 
-template <typename OT>
-__global__ void noise_fill_kernel(OT* __restrict__ out, int64_t N, double scale, uint64_t step,
-                                  uint64_t mul, uint64_t seed, int component) {
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        double u1, u2;
-        hash_pair(noise_key((uint64_t)s, step, mul, seed), u1, u2);
-        double r = bm_radius(u1);
-        double v = component ? r * sin(kTwoPiLit * u2) : r * cos(kTwoPiLit * u2);
-        out[s] = (OT)(scale * v);
+// Two sites a thread and pass: the transform's constants are loaded once for both
+// (146 thread instructions a site instead of 166 with one site, 233 with CUDA's log,
+// sqrt and cos).  256^3 float32: 142 us with those, 105 us with one site, 98 us here.
+template <typename OT, bool SIN>
+__global__ void __launch_bounds__(256) noise_fill_kernel(OT* __restrict__ out, int64_t N,
+                                                         double scale, uint64_t step, uint64_t mul,
+                                                         uint64_t seed) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N; s += 2 * stride) {
+        const uint64_t k0 = noise_key((uint64_t)s, step, mul, seed);
+        const uint64_t k1 = noise_key((uint64_t)(s + stride), step, mul, seed);
+        const double z0 = SIN ? gauss_sin(k0) : gauss_cos(k0);
+        const double z1 = SIN ? gauss_sin(k1) : gauss_cos(k1);
+        out[s] = (OT)__dmul_rn(scale, z0);
+        if (s + stride < N) out[s + stride] = (OT)__dmul_rn(scale, z1);
     }
 }
 
@@ -49,12 +56,13 @@ int launch_hash_pairs(const uint64_t* keys, int64_t n, double* u1, double* u2, d
 int launch_noise_fill(int storage, void* out, int64_t N, double scale, uint64_t step,
                       uint64_t mul, uint64_t seed, int component, cudaStream_t st) {
     if (N == 0) return TIPT_OK;
-    if (storage == TIPT_F64)
-        noise_fill_kernel<double><<<grid_for(N, 256), 256, 0, st>>>(
-            static_cast<double*>(out), N, scale, step, mul, seed, component);
-    else
-        noise_fill_kernel<float><<<grid_for(N, 256), 256, 0, st>>>(
-            static_cast<float*>(out), N, scale, step, mul, seed, component);
+    const unsigned g = grid_for((N + 1) / 2, 256);
+    const auto fill = [&](auto* o) {
+        if (component) noise_fill_kernel<std::remove_pointer_t<decltype(o)>, true><<<g, 256, 0, st>>>(o, N, scale, step, mul, seed);
+        else noise_fill_kernel<std::remove_pointer_t<decltype(o)>, false><<<g, 256, 0, st>>>(o, N, scale, step, mul, seed);
+    };
+    if (storage == TIPT_F64) fill(static_cast<double*>(out));
+    else fill(static_cast<float*>(out));
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "noise_fill launch");
 }

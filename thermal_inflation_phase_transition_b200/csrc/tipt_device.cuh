@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "gauss64.cuh"
 #include "tipt.h"
 
 namespace tipt {
@@ -16,7 +17,6 @@ namespace tipt {
 constexpr uint64_t kPass2Mul = 73856093ull;   // R:2518 (pass 2 / midpoint)
 constexpr uint64_t kPass4Mul = 19349669ull;   // R:2643 (pass 4)
 constexpr uint64_t kSeedStride = 0x9E3779B97F4A7C15ull;
-constexpr double kTwoPiLit = 6.283185307179586;  // literal of R:2520
 
 // Order-preserving integer code of a float (unsigned comparison = float order).
 __device__ __forceinline__ unsigned int ord_code(float f) {
@@ -76,15 +76,24 @@ __device__ __forceinline__ void reset_range_words(unsigned int* next) {
 // ---------------------------------------------------------------- noise ----
 // R:2322-2336 _hash_rng_pair: splitmix-style mix -> two 53-bit uniforms.  The
 // second mix of the reference kernel is partial (no >>27 round); u1 >= 1e-12.
-__device__ __forceinline__ void hash_pair(uint64_t x, double& u1, double& u2) {
+// hash_bits gives the 53-bit integers m1, m2 (u = m 2^-53, u1 not yet clamped).
+__device__ __forceinline__ void hash_bits(uint64_t x, uint64_t& m1, uint64_t& m2) {
     x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
     x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
     x = x ^ (x >> 31);
-    u1 = (double)(x >> 11) * (1.0 / 9007199254740992.0);
-    x = (x * 0x2545F4914F6CDD1Dull) ^ 0x9E3779B97F4A7C15ull;
-    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
+    m1 = x >> 11;
+    // (y ^ C) ^ ((y ^ C) >> 30) = y ^ (y >> 30) ^ (C ^ (C >> 30)): one xor fewer
+    constexpr uint64_t kC = 0x9E3779B97F4A7C15ull, kCs = kC ^ (kC >> 30);
+    x = x * 0x2545F4914F6CDD1Dull;
+    x = (x ^ (x >> 30) ^ kCs) * 0xBF58476D1CE4E5B9ull;
     x = x ^ (x >> 31);
-    u2 = (double)(x >> 11) * (1.0 / 9007199254740992.0);
+    m2 = x >> 11;
+}
+__device__ __forceinline__ void hash_pair(uint64_t x, double& u1, double& u2) {
+    uint64_t m1, m2;
+    hash_bits(x, m1, m2);
+    u1 = (double)m1 * (1.0 / 9007199254740992.0);
+    u2 = (double)m2 * (1.0 / 9007199254740992.0);
     u1 = u1 < 1e-12 ? 1e-12 : u1;
 }
 
@@ -99,22 +108,33 @@ __device__ __forceinline__ uint64_t noise_key(uint64_t site, uint64_t step, uint
     return (sm ^ step) + seed * kSeedStride;
 }
 
-// R:2519-2521 Box-Muller radius and angle, FP64 (the reference's precision).
-__device__ __forceinline__ double bm_radius(double u1) { return sqrt(-2.0 * log(u1)); }
+// R:2519-2521 Box-Muller in FP64 (the reference's precision), gauss64.cuh.
 __device__ __forceinline__ double gauss_cos(uint64_t key) {
-    double u1, u2;
-    hash_pair(key, u1, u2);
-    return bm_radius(u1) * cos(kTwoPiLit * u2);
+    uint64_t m1, m2;
+    hash_bits(key, m1, m2);
+    double s, d;
+    sqrt_parts(neg2_log_m(m1), s, d);
+    const double c = cos_m(angle_m(m2), m2);
+    return __fma_rn(s, c, __dmul_rn(d, c));
+}
+__device__ __forceinline__ double gauss_sin(uint64_t key) {
+    uint64_t m1, m2;
+    hash_bits(key, m1, m2);
+    double s, d;
+    sqrt_parts(neg2_log_m(m1), s, d);
+    const double c = sin_m(angle_m(m2), m2);
+    return __fma_rn(s, c, __dmul_rn(d, c));
 }
 // C:2965-2970: the complex field draws one pair per site: cos -> pi1, sin -> pi2.
 __device__ __forceinline__ void gauss_pair(uint64_t key, double& z1, double& z2) {
-    double u1, u2;
-    hash_pair(key, u1, u2);
-    double r = bm_radius(u1);
-    double s, c;
-    sincos(kTwoPiLit * u2, &s, &c);
-    z1 = r * c;
-    z2 = r * s;
+    uint64_t m1, m2;
+    hash_bits(key, m1, m2);
+    double s, d;
+    sqrt_parts(neg2_log_m(m1), s, d);
+    const double a = angle_m(m2);
+    const double c = cos_m(a, m2), sn = sin_m(a, m2);
+    z1 = __fma_rn(s, c, __dmul_rn(d, c));
+    z2 = __fma_rn(s, sn, __dmul_rn(d, sn));
 }
 
 // ------------------------------------------------ FP32 lane vectors ----
