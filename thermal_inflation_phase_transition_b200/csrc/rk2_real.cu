@@ -6,101 +6,10 @@
 //  * rk2_stage_march (rk2_march.cuh): the bandwidth kernel for n2 % 4 == 0.
 #include "rk2_real.cuh"
 #include "rk2_march.cuh"
+#include "stage_kernels.cuh"
 #include "tipt_internal.h"
 
 namespace tipt {
-
-template <int S, bool TH, bool RG>
-__global__ void __launch_bounds__(256) rk2_stage_generic(RealStageParams p_in) {
-    RealStageParams p = p_in;
-    resolve_schedule(p);
-    if constexpr (RG) reset_next_range(p);
-    RangeAcc racc;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    using TT = typename std::conditional<S == TIPT_F32C, float, double>::type;
-    TT* s_tab = reinterpret_cast<TT*>(smem_raw);
-    if (p.table_in_smem) stage_table<TT>(p, s_tab);
-    const F32CConst kc = f32c_const(p);
-
-    const int64_t n12 = (int64_t)p.n1 * p.n2;
-    const int64_t N = (int64_t)p.n0 * n12;
-    const int64_t s_end = (int64_t)p.i_end * n12;
-    for (int64_t s = (int64_t)p.i_begin * n12 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-         s < s_end; s += (int64_t)gridDim.x * blockDim.x) {
-        const int k = (int)(s % p.n2);
-        const int64_t r = s / p.n2;
-        const int j = (int)(r % p.n1);
-        const int i = (int)(r / p.n1);
-        const int64_t o_ip = (i + 1 < p.n0) ? n12 : -(int64_t)(p.n0 - 1) * n12;
-        const int64_t o_im = (i > 0) ? -n12 : (int64_t)(p.n0 - 1) * n12;
-        const int64_t o_jp = (j + 1 < p.n1) ? p.n2 : -(int64_t)(p.n1 - 1) * p.n2;
-        const int64_t o_jm = (j > 0) ? -(int64_t)p.n2 : (int64_t)(p.n1 - 1) * p.n2;
-        const int64_t o_kp = (k + 1 < p.n2) ? 1 : -(int64_t)(p.n2 - 1);
-        const int64_t o_km = (k > 0) ? -1 : (int64_t)(p.n2 - 1);
-        const int64_t idx[7] = {s, s + o_ip, s + o_im, s + o_jp, s + o_jm, s + o_kp, s + o_km};
-        if constexpr (S == TIPT_F64) {
-            const double* phi = static_cast<const double*>(p.phi);
-            const double* pi = static_cast<const double*>(p.pi);
-            double ph[7], pv[7];
-#pragma unroll
-            for (int q = 0; q < 7; ++q) {
-                ph[q] = __ldg(phi + idx[q]);
-                pv[q] = __ldg(pi + idx[q]);
-            }
-            double a, b;
-            update_f64<TH>(p, reinterpret_cast<const double*>(s_tab), ph, pv,
-                       site_noise<double>(p, (uint64_t)(s + p.site_offset)), a, b);
-            static_cast<double*>(p.phi_out)[s] = a;
-            static_cast<double*>(p.pi_out)[s] = b;
-            if constexpr (RG) racc.fold_d(a);
-        } else if constexpr (S == TIPT_F32) {
-            const float* phi = static_cast<const float*>(p.phi);
-            const float* pi = static_cast<const float*>(p.pi);
-            float ph[7], pv[7];
-#pragma unroll
-            for (int q = 0; q < 7; ++q) {
-                ph[q] = __ldg(phi + idx[q]);
-                pv[q] = __ldg(pi + idx[q]);
-            }
-            float a, b;
-            update_f32<TH>(p, reinterpret_cast<const double*>(s_tab), ph, pv,
-                       site_noise<float>(p, (uint64_t)(s + p.site_offset)), a, b);
-            static_cast<float*>(p.phi_out)[s] = a;
-            static_cast<float*>(p.pi_out)[s] = b;
-            if constexpr (RG) racc.fold(a);
-        } else {
-            // planar {hi, lo}: hi plane at [0, N), lo plane at [N, 2N)
-            const float* phi = static_cast<const float*>(p.phi);
-            const float* pi = static_cast<const float*>(p.pi);
-            float hh[7], hl[7], vh[7], vl[7];
-#pragma unroll
-            for (int q = 0; q < 7; ++q) {
-                hh[q] = __ldg(phi + idx[q]);
-                hl[q] = __ldg(phi + N + idx[q]);
-                vh[q] = __ldg(pi + idx[q]);
-                vl[q] = __ldg(pi + N + idx[q]);
-            }
-            F32CIn<float> x;
-            stencil_sums_k(hh, hl, x.dh_phi, x.dl_phi);
-            stencil_sums_k(vh, vl, x.dh_pi, x.dl_pi);
-            x.phh = hh[0];
-            x.phl = hl[0];
-            x.pih = vh[0];
-            x.pil = vl[0];
-            float a, b, c, d;
-            update_f32c<float, TH>(p, kc, reinterpret_cast<const float*>(s_tab), x,
-                               site_kick_f32c(p, kc, (uint64_t)(s + p.site_offset)), a, b, c, d);
-            float* po = static_cast<float*>(p.phi_out);
-            float* vo = static_cast<float*>(p.pi_out);
-            po[s] = a;
-            po[N + s] = b;
-            vo[s] = c;
-            vo[N + s] = d;
-            if constexpr (RG) racc.fold_ff(a, b);
-        }
-    }
-    if constexpr (RG) racc.flush(p.range);
-}
 
 // Bytes of shared memory the V' row needs for storage S (0 if polynomial).
 static int64_t table_smem_bytes(int S, const RealStageParams& p) {
@@ -120,22 +29,10 @@ int num_sms() {
 }
 
 template <int S>
-static int launch_generic(RealStageParams p, int64_t smem, cudaStream_t st) {
-    auto kern = p.vkind == TIPT_VP_THERMAL
-                    ? (p.range ? rk2_stage_generic<S, true, true> : rk2_stage_generic<S, true, false>)
-                    : (p.range ? rk2_stage_generic<S, false, true> : rk2_stage_generic<S, false, false>);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return fail_cuda(e, "rk2_stage_generic smem attribute");
-    }
-    const int64_t N = (int64_t)(p.i_end - p.i_begin) * p.n1 * p.n2;
-    int64_t blocks = (N + 255) / 256;
-    const int64_t cap = (int64_t)num_sms() * 8;
-    if (blocks > cap) blocks = cap;
-    kern<<<(unsigned)blocks, 256, (size_t)smem, st>>>(p);
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "rk2_stage_generic launch");
+static int launch_generic(const RealStageParams& p, int64_t smem, cudaStream_t st) {
+    const bool th = p.vkind == TIPT_VP_THERMAL;
+    if (p.range) return th ? launch_stage_generic<RealSite<S, true, true>>(p, smem, st) : launch_stage_generic<RealSite<S, false, true>>(p, smem, st);
+    return th ? launch_stage_generic<RealSite<S, true, false>>(p, smem, st) : launch_stage_generic<RealSite<S, false, false>>(p, smem, st);
 }
 
 // Largest V' row staged in shared memory; longer 1-D tables are read from

@@ -271,48 +271,48 @@ __device__ __forceinline__ double sum6_d(const double v[7]) {
     return __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(v[1], v[2]), v[3]), v[4]), v[5]), v[6]);
 }
 __device__ __forceinline__ double force_d(const RealStageParams& p, double lap, double pv, double dv) {
-    // inv_a2*lap - eta*pi - V'/mu^2
-    return __dsub_rn(__dsub_rn(__dmul_rn(p.inv_a2, lap), __dmul_rn(p.eta, pv)), __dmul_rn(dv, p.inv_mu2));
+    // inv_a2*lap - eta*pi - V'/mu^2 as two fused multiply-adds
+    return __fma_rn(-dv, p.inv_mu2, __fma_rn(-p.eta, pv, __dmul_rn(p.inv_a2, lap)));
 }
+// phi~ = phi + h1 pi is linear in the state, so its Laplacian is lap + h1 lap(pi): no
+// midpoint value per neighbour.
 template <bool TH = true>
 __device__ __forceinline__ void update_f64(const RealStageParams& p, const double* s_tab,
                                            const double ph[7], const double pv[7], double noise,
                                            double& phi_new, double& pi_new) {
     const double c = ph[0];
     const double lap = __dmul_rn(__fma_rn(-6.0, c, sum6_d(ph)), p.inv_dx2);
-    double pt[7];
-#pragma unroll
-    for (int q = 0; q < 7; ++q) pt[q] = __fma_rn(p.h1, pv[q], ph[q]);
-    const double lap2 = __dmul_rn(__fma_rn(-6.0, pt[0], sum6_d(pt)), p.inv_dx2);
+    const double lapv = __dmul_rn(__fma_rn(-6.0, pv[0], sum6_d(pv)), p.inv_dx2);
     const double k1 = force_d(p, lap, pv[0], vprime_d<TH>(p, s_tab, c));
     const double pit = __fma_rn(p.h1, k1, pv[0]);
-    const double k2 = force_d(p, lap2, pit, vprime_d<TH>(p, s_tab, pt[0]));
+    const double k2 = force_d(p, __fma_rn(p.h1, lapv, lap), pit,
+                              vprime_d<TH>(p, s_tab, __fma_rn(p.h1, pv[0], c)));
     phi_new = __fma_rn(p.h2, pit, c);
     pi_new = __dadd_rn(pv[0], __fma_rn(p.h2, k2, noise));
 }
 
 // --------------------------------------------------------------- F32 ----
-// The reference's float32 mode (USE_FLOAT32, R:348): float32 neighbour sums,
-// FP64 for the rest, float32 stores -- including the stored midpoint state
-// phi~, pi~ that pass 2 reads (R:1932-1933).
+// The reference's float32 mode (USE_FLOAT32, R:348): float32 neighbour sums, FP64
+// for the rest, float32 stores, among them the midpoint's pi~ (R:1933).  The
+// midpoint's phi~ stays in FP64: the reference rounds it to float32 at every
+// neighbour (R:1932), which here would be 27 conversions between FP32 and FP64 a
+// site (their unit bound the stage) for a less exact Laplacian.
+__device__ __forceinline__ float sum6_f(const float v[7]) {
+    return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(v[1], v[2]), v[3]), v[4]), v[5]), v[6]);
+}
 template <bool TH = true>
 __device__ __forceinline__ void update_f32(const RealStageParams& p, const double* s_tab,
                                            const float ph[7], const float pv[7], double noise,
                                            float& phi_new, float& pi_new) {
-    const float c = ph[0];
-    float s6 = ph[1] + ph[2] + ph[3] + ph[4] + ph[5] + ph[6];
-    double lap = ((double)s6 - 6.0 * (double)c) * p.inv_dx2;
-    float pt[7];
-#pragma unroll
-    for (int q = 0; q < 7; ++q) pt[q] = __double2float_rn((double)ph[q] + p.h1 * (double)pv[q]);
-    float s6b = pt[1] + pt[2] + pt[3] + pt[4] + pt[5] + pt[6];
-    double lap2 = ((double)s6b - 6.0 * (double)pt[0]) * p.inv_dx2;
-    double k1 = p.inv_a2 * lap - p.eta * (double)pv[0] - vprime_d<TH>(p, s_tab, (double)c) * p.inv_mu2;
-    float pit = __double2float_rn((double)pv[0] + p.h1 * k1);
-    double k2 = p.inv_a2 * lap2 - p.eta * (double)pit -
-                vprime_d<TH>(p, s_tab, (double)pt[0]) * p.inv_mu2;
-    phi_new = __double2float_rn((double)c + p.h2 * (double)pit);
-    pi_new = __double2float_rn((double)pv[0] + (p.h2 * k2 + noise));
+    const double c = (double)ph[0], v = (double)pv[0];
+    const double lap = __dmul_rn(__fma_rn(-6.0, c, (double)sum6_f(ph)), p.inv_dx2);
+    const double lapv = __dmul_rn(__fma_rn(-6.0, v, (double)sum6_f(pv)), p.inv_dx2);
+    const double k1 = force_d(p, lap, v, vprime_d<TH>(p, s_tab, c));
+    const double pit = (double)__double2float_rn(__fma_rn(p.h1, k1, v));
+    const double k2 = force_d(p, __fma_rn(p.h1, lapv, lap), pit,
+                              vprime_d<TH>(p, s_tab, __fma_rn(p.h1, v, c)));
+    phi_new = __double2float_rn(__fma_rn(p.h2, pit, c));
+    pi_new = __double2float_rn(__dadd_rn(v, __fma_rn(p.h2, k2, noise)));
 }
 
 // -------------------------------------------------------------- F32C ----
