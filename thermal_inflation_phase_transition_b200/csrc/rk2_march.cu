@@ -29,6 +29,8 @@
 // producer drains the copies it issued (bounded) before it exits.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "integrators.cuh"
 #include "rk2_march.cuh"
 #include "tipt_internal.h"
@@ -128,10 +130,10 @@ struct MarchGeom {
     int items;
     int tab_bytes;    // staged V' row (bytes, 128-aligned)
     int stage_bytes;  // one ring stage: phi and pi tiles
-    // compensated-FP32 single-lattice stage only: 1 = each CTA takes an equal
-    // share of the nJB x planes (j-block, plane) units, j-block major, as one or
-    // more runs of planes (items is then the number of units); 0 = items of CI
-    // planes.  Every geometry starts with 0; only launch_f32c_stage sets it.
+    // 1 = each CTA takes an equal share of the (tile, plane) units, tile major, as
+    // one or more runs of planes (items is then the number of units); 0 = items of
+    // CI planes.  Every geometry starts with 0; split_work sets it at the launch (not
+    // for the items of a batched ensemble).
     int bal = 0;
     // complex kernel: rows split into nKS segments of KS sites (with nKS > 1 the
     // k-1 / k+1 neighbours of a segment's end sites are copied by the edge
@@ -217,6 +219,54 @@ struct RingPos {
 // 17-18 warps per SM must fit the four 16K-register sub-partitions.
 constexpr int kMarchRegs = 96;
 
+// The (tile, first plane, planes) runs of one CTA, walked alike by producer and
+// consumers.  MarchGeom::bal = 0: items of CI planes, round robin, tiles innermost, so
+// that the CTAs of neighbouring tiles are at the same planes.  bal = 1: CTA b of G takes
+// the units [U b / G, U (b + 1) / G) of the U = tiles x planes (tile, plane) units, tile
+// major, split where a tile ends.
+// Only the producer walks them: it hands every run to the consumers through a slot in
+// shared memory, written before the run's first plane is announced (the arrival on its
+// full barrier orders the two), so the consumers' plane loop carries no walk (which
+// cost the complex stage at 256^3 8 %, short of registers as it is).  Two slots: when a
+// stage is free for the first plane of run r + 2, every warp has released a plane five
+// positions back at least, which is one of run r or r + 1 (a run has three planes or
+// more, a ring at most five stages), so it has read slot r.
+struct MarchRuns {
+    int u, end;
+    __device__ __forceinline__ MarchRuns(const MarchGeom& g, int tiles, int npl) {
+        u = blockIdx.x;
+        end = g.items;
+        if (g.bal) {
+            const int64_t U = (int64_t)tiles * npl;
+            u = (int)(U * blockIdx.x / gridDim.x);
+            end = (int)(U * (blockIdx.x + 1) / gridDim.x);
+        }
+    }
+    __device__ __forceinline__ bool more() const { return u < end; }
+    __device__ __forceinline__ void next(const MarchGeom& g, int tiles, int i_begin, int i_end,
+                                         int& tile, int& i0, int& ni) {
+        const int npl = i_end - i_begin;
+        if (g.bal) {
+            tile = u / npl;
+            const int off = u - tile * npl;
+            ni = min(npl - off, end - u);
+            i0 = i_begin + off;
+            u += ni;
+        } else {
+            const int ic = u / tiles;
+            tile = u - ic * tiles;
+            i0 = i_begin + ic * g.CI;
+            ni = min(g.CI, i_end - i0);
+            u += gridDim.x;
+        }
+    }
+};
+// The slots lie in the header's unused barrier words: full[6..7] and empty[6..7]
+// (`full` points at sixteen words, `empty` at its second half).
+__device__ __forceinline__ int4* run_slot(uint64_t* full, int run) {
+    return reinterpret_cast<int4*>(full + 6 + 8 * (run & 1));
+}
+
 template <int S, bool WIDE>
 __global__ void __maxnreg__(kMarchRegs)
     rk2_stage_march(RealStageParams p_in, MarchGeom g) {
@@ -267,16 +317,19 @@ __global__ void __maxnreg__(kMarchRegs)
         RingPos w{0, 0};
         uint32_t issued = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < g.items && ok; item += gridDim.x) {
-            const int ic = item / g.nJB;
-            const int j0 = (item - ic * g.nJB) * TJ, i0 = p.i_begin + ic * g.CI;
-            const int npl = min(g.CI, p.i_end - i0) + 2;
+        int run = 0;
+        for (MarchRuns runs(g, g.nJB, p.i_end - p.i_begin); runs.more() && ok; ++run) {
+            int j0, i0, ni;
+            runs.next(g, g.nJB, p.i_begin, p.i_end, j0, i0, ni);
+            j0 *= TJ;
+            const int npl = ni + 2;
             for (int q = 0; q < npl; ++q) {
                 // stage w.stage last held position issued - NS, released in phase w.phase ^ 1
                 if (issued >= NS && !mbar_wait(&empty[w.stage], w.phase ^ 1u)) {
                     ok = false;
                     break;
                 }
+                if (q == 0) *run_slot(full, run) = make_int4(j0, i0, ni, runs.more());
                 mbar_expect_tx(&full[w.stage], plane_tx);
                 int iw = i0 - 1 + q;
                 iw = iw < 0 ? iw + n0 : (iw >= n0 ? iw - n0 : iw);
@@ -313,11 +366,7 @@ __global__ void __maxnreg__(kMarchRegs)
     const int orow = r * pitch, urow = (r - 1) * pitch, drow = (r + 1) * pitch;
 
     RingPos pm{0, 0};  // ring position of plane i-1 for the current iteration
-    for (int item = blockIdx.x; item < g.items; item += gridDim.x) {
-        const int ic = item / g.nJB;
-        const int j0 = (item - ic * g.nJB) * TJ, i0 = p.i_begin + ic * g.CI;
-        const int ni = min(g.CI, p.i_end - i0);
-        const int jw = j0 + r - 1;
+    for (int run = 0, more = 1; more; ++run) {
         RingPos pc = pm, pp;
         pc.next(NS);
         pp = pc;
@@ -326,6 +375,9 @@ __global__ void __maxnreg__(kMarchRegs)
             if (lane == 0) atomicExch(&g_device_status, (int)TIPT_ERR_TIMEOUT);
             return;
         }
+        const int4 rs = *run_slot(full, run);
+        const int jw = rs.x + r - 1, i0 = rs.y, ni = rs.z;
+        more = rs.w;
         for (int q = 0; q < ni; ++q) {
             const int i = i0 + q;
             const int64_t rowoff = ((int64_t)i * n1 + jw) * n2;
@@ -406,30 +458,6 @@ struct EnsMarch {
     uint64_t step;
     const unsigned long long* ctr;  // device step counter or nullptr
     long long offset;
-};
-
-// The runs of planes of one CTA under MarchGeom::bal: CTA b of G takes the units
-// [U b / G, U (b + 1) / G) of the U = nJB x planes (j-block, plane) units, j-block
-// major, split where a j-block ends.  Producer and consumers walk the same runs.
-struct BalRun {
-    int64_t u, u_end;
-    int npl, i_begin;
-    __device__ __forceinline__ BalRun(const MarchGeom& g, const RealStageParams& p, int b, int G) {
-        npl = p.i_end - p.i_begin;
-        i_begin = p.i_begin;
-        const int64_t U = (int64_t)g.nJB * npl;
-        u = g.bal ? U * b / G : 0;
-        u_end = g.bal ? U * (b + 1) / G : 0;
-    }
-    __device__ __forceinline__ bool more() const { return u < u_end; }
-    // the next run: j-block jb, first plane i0, ni planes
-    __device__ __forceinline__ void next(int& jb, int& i0, int& ni) {
-        jb = (int)(u / npl);
-        const int off = (int)(u - (int64_t)jb * npl);
-        ni = (int)min((int64_t)(npl - off), u_end - u);
-        i0 = i_begin + off;
-        u += ni;
-    }
 };
 
 // Planar compensated-FP32 marching kernel.  Same ring, roles and work items as
@@ -518,10 +546,11 @@ __global__ void __maxnreg__(kMarchRegs)
         if constexpr (ENS) {
             if (em.n_rids) n_items = min(g.items, *em.n_rids * em.items_per_rep);
         }
-        BalRun br(g, p, blockIdx.x, gridDim.x);
-        for (int item = blockIdx.x; ((!ENS && g.bal) ? br.more() : item < n_items) && ok;
-             item += gridDim.x) {
-            int it = item;
+        MarchRuns runs(g, g.nJB, p.i_end - p.i_begin);
+        int run = 0;
+        for (int item = blockIdx.x; (ENS ? item < n_items : runs.more()) && ok;
+             item += gridDim.x, ++run) {
+            int it = 0;
             const float *phi_hi = src_phi, *phi_lo = src_phi + plane_n;
             const float *pi_hi = src_pi, *pi_lo = src_pi + plane_n;
             if constexpr (ENS) {
@@ -540,14 +569,14 @@ __global__ void __maxnreg__(kMarchRegs)
                 pi_lo = src_pi + em.n_total + off;
             }
             int j0, i0, ni;
-            if (!ENS && g.bal) {
-                br.next(j0, i0, ni);
-                j0 *= TJ;
-            } else {
+            if constexpr (ENS) {
                 const int ic = it / g.nJB;
                 j0 = (it - ic * g.nJB) * TJ;
                 i0 = p.i_begin + ic * g.CI;
                 ni = min(g.CI, p.i_end - i0);
+            } else {
+                runs.next(g, g.nJB, p.i_begin, p.i_end, j0, i0, ni);
+                j0 *= TJ;
             }
             const int npl = ni + 2;
             for (int q = 0; q < npl; ++q) {
@@ -559,6 +588,7 @@ __global__ void __maxnreg__(kMarchRegs)
                     ok = false;
                     break;
                 }
+                if (!ENS && q == 0) *run_slot(full, run) = make_int4(j0, i0, ni, runs.more());
                 mbar_expect_tx(&full[w.stage], plane_tx);
                 int iw = i0 - 1 + q;
                 iw = iw < 0 ? iw + n0 : (iw >= n0 ? iw - n0 : iw);
@@ -605,9 +635,9 @@ __global__ void __maxnreg__(kMarchRegs)
     if constexpr (ENS) {
         if (em.n_rids) n_items = min(g.items, *em.n_rids * em.items_per_rep);
     }
-    BalRun br(g, p, blockIdx.x, gridDim.x);  // the producer's sequence of runs
-    for (int item = blockIdx.x; (!ENS && g.bal) ? br.more() : item < n_items; item += gridDim.x) {
-        int it = item;
+    int run = 0, more = 1;
+    for (int item = blockIdx.x; ENS ? item < n_items : more; item += gridDim.x, ++run) {
+        int it = 0;
         if constexpr (ENS) {
             const int rl = item / em.items_per_rep;
             const int rid = em.rids[rl];
@@ -625,17 +655,6 @@ __global__ void __maxnreg__(kMarchRegs)
             kc.ns = (float)rp.noise_scale;
             eseed = rp.seed;
         }
-        int j0, i0, ni;
-        if (!ENS && g.bal) {
-            br.next(j0, i0, ni);
-            j0 *= TJ;
-        } else {
-            const int ic = it / g.nJB;
-            j0 = (it - ic * g.nJB) * TJ;
-            i0 = p.i_begin + ic * g.CI;
-            ni = min(g.CI, p.i_end - i0);
-        }
-        const int jw = j0 + r - 1;
         RingPos pc = pm, pp;
         pc.next(NS);
         pp = pc;
@@ -644,6 +663,20 @@ __global__ void __maxnreg__(kMarchRegs)
             if (lane == 0) atomicExch(&g_device_status, (int)TIPT_ERR_TIMEOUT);
             return;
         }
+        int j0, i0, ni;
+        if constexpr (ENS) {
+            const int ic = it / g.nJB;
+            j0 = (it - ic * g.nJB) * TJ;
+            i0 = p.i_begin + ic * g.CI;
+            ni = min(g.CI, p.i_end - i0);
+        } else {
+            const int4 rs = *run_slot(full, run);
+            j0 = rs.x;
+            i0 = rs.y;
+            ni = rs.z;
+            more = rs.w;
+        }
+        const int jw = j0 + r - 1;
         for (int q = 0; q < ni; ++q) {
             const int i = i0 + q;
             const int64_t rowoff = ((int64_t)i * n1 + jw) * n2 + k0;
@@ -847,15 +880,18 @@ __global__ void __maxnreg__(kMarchRegs) alt_march_f32c(AltParams p, MarchGeom g)
         RingPos w{0, 0};
         uint32_t issued = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < g.items && ok; item += gridDim.x) {
-            const int ic = item / g.nJB;
-            const int j0 = (item - ic * g.nJB) * TJ, i0 = ic * g.CI;
-            const int npl = min(g.CI, n0 - i0) + 2;
+        int run = 0;
+        for (MarchRuns runs(g, g.nJB, n0); runs.more() && ok; ++run) {
+            int j0, i0, ni;
+            runs.next(g, g.nJB, 0, n0, j0, i0, ni);
+            j0 *= TJ;
+            const int npl = ni + 2;
             for (int q = 0; q < npl; ++q) {
                 if (issued >= NS && !mbar_wait(&empty[w.stage], w.phase ^ 1u)) {
                     ok = false;
                     break;
                 }
+                if (q == 0) *run_slot(full, run) = make_int4(j0, i0, ni, runs.more());
                 mbar_expect_tx(&full[w.stage], plane_tx);
                 int iw = i0 - 1 + q;
                 iw = iw < 0 ? iw + n0 : (iw >= n0 ? iw - n0 : iw);
@@ -892,11 +928,7 @@ __global__ void __maxnreg__(kMarchRegs) alt_march_f32c(AltParams p, MarchGeom g)
     const float tminf = (float)p.v.tmin, dinvf = (float)p.v.dinv, last = (float)(p.v.npts - 2);
 
     RingPos pm{0, 0};
-    for (int item = blockIdx.x; item < g.items; item += gridDim.x) {
-        const int ic = item / g.nJB;
-        const int j0 = (item - ic * g.nJB) * TJ, i0 = ic * g.CI;
-        const int ni = min(g.CI, n0 - i0);
-        const int jw = j0 + r - 1;
+    for (int run = 0, more = 1; more; ++run) {
         RingPos pc = pm, pp;
         pc.next(NS);
         pp = pc;
@@ -905,6 +937,9 @@ __global__ void __maxnreg__(kMarchRegs) alt_march_f32c(AltParams p, MarchGeom g)
             if (lane == 0) atomicExch(&g_device_status, (int)TIPT_ERR_TIMEOUT);
             return;
         }
+        const int4 rs = *run_slot(full, run);
+        const int jw = rs.x + r - 1, i0 = rs.y, ni = rs.z;
+        more = rs.w;
         for (int q = 0; q < ni; ++q) {
             const int64_t rowoff = ((int64_t)(i0 + q) * n1 + jw) * n2 + k0;
             // pi at the thread's own four sites (BAOAB passes), loaded before the
@@ -1058,7 +1093,12 @@ __global__ void __maxnreg__(kMarchRegs) alt_march_f32c(AltParams p, MarchGeom g)
 // KKS, KTJ > 0: segments of KKS sites (pitch KKS) in KTJ-row tiles fixed at
 // compile time, as the real stage's fixed geometry (the launcher takes it when
 // the run-time geometry is exactly that one).
-template <bool WIDE, bool RG, int KKS = 0, int KTJ = 0>
+//
+// BAL: equal shares of the work (MarchGeom::bal), the runs handed over through the
+// slots.  Without it both roles walk the items from blockIdx alone, which keeps the
+// coordinates of the tensor copies in uniform registers: with the two forms chosen at
+// run time the producer's issue bound the stage (512^3 2.17 -> 2.67 ms).
+template <bool WIDE, bool RG, bool BAL, int KKS = 0, int KTJ = 0>
 __global__ void __maxnreg__(kMarchRegs)
     complex_stage_march_f32c(const __grid_constant__ CUtensorMap tm0,
                              const __grid_constant__ CUtensorMap tm1,
@@ -1119,32 +1159,55 @@ __global__ void __maxnreg__(kMarchRegs)
         RingPos w{0, 0};
         uint32_t issued = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < g.items && ok; item += gridDim.x) {
-            const int ic = item / nJK;
-            const int jk = item - ic * nJK;
+        MarchRuns runs(g, nJK, n0);
+        int run = 0;
+        for (int item = blockIdx.x; (BAL ? runs.more() : item < g.items) && ok;
+             item += gridDim.x, ++run) {
+            int jk, i0, ni;
+            if constexpr (BAL) {
+                runs.next(g, nJK, 0, n0, jk, i0, ni);
+            } else {
+                const int ic = item / nJK;
+                jk = item - ic * nJK;
+                i0 = ic * g.CI;
+                ni = min(g.CI, n0 - i0);
+            }
             const int jb = jk / g.nKS;
             const int k0s = (jk - jb * g.nKS) * KS;
-            const int j0 = jb * TJ, i0 = ic * g.CI;
-            const int npl = min(g.CI, n0 - i0) + 2;
+            const int j0 = jb * TJ;
+            const int npl = ni + 2;
             for (int q = 0; q < npl; ++q) {
                 if (issued >= NS && !mbar_wait(&empty[w.stage], w.phase ^ 1u)) {
                     ok = false;
                     break;
                 }
+                if (BAL && q == 0) *run_slot(full, run) = make_int4(jk, i0, ni, runs.more());
                 mbar_expect_tx(&full[w.stage], plane_tx);
                 int iw = i0 - 1 + q;
                 iw = iw < 0 ? iw + n0 : (iw >= n0 ? iw - n0 : iw);
-                for (int rr = 0; rr < rows; ++rr) {
-                    int jr = j0 - 1 + rr;
-                    jr = jr < 0 ? jr + n1 : (jr >= n1 ? jr - n1 : jr);
-                    for (int kb = 0; kb < KS; kb += g.BK) {
-                        const int o = rr * pitch + kb;
+                if (!split && pitch == n2) {
+                    // whole rows: one bulk copy per run of consecutive rows (at most three
+                    // a component where the tile wraps in j), not one box per row: 8
+                    // copies a plane instead of 8 (TJ + 2), whose issue bound the stage
 #pragma unroll
-                        for (int f = 0; f < 4; ++f) {
-                            // plane iw = hi, plane n0 + iw = lo
-                            tma_row(blk(w.stage, f, 0) + o, tm[f], k0s + kb, jr, iw, &full[w.stage]);
-                            tma_row(blk(w.stage, f, 1) + o, tm[f], k0s + kb, jr, n0 + iw,
-                                    &full[w.stage]);
+                    for (int f = 0; f < 4; ++f)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+                            copy_tile_rows(blk(w.stage, f, c), static_cast<const float*>(p.f[f]),
+                                           iw + c * n0, j0, rows, n1, n2, pitch, &full[w.stage]);
+                } else {
+                    for (int rr = 0; rr < rows; ++rr) {
+                        int jr = j0 - 1 + rr;
+                        jr = jr < 0 ? jr + n1 : (jr >= n1 ? jr - n1 : jr);
+                        for (int kb = 0; kb < KS; kb += g.BK) {
+                            const int o = rr * pitch + kb;
+#pragma unroll
+                            for (int f = 0; f < 4; ++f) {
+                                // plane iw = hi, plane n0 + iw = lo
+                                tma_row(blk(w.stage, f, 0) + o, tm[f], k0s + kb, jr, iw, &full[w.stage]);
+                                tma_row(blk(w.stage, f, 1) + o, tm[f], k0s + kb, jr, n0 + iw,
+                                        &full[w.stage]);
+                            }
                         }
                     }
                 }
@@ -1195,21 +1258,35 @@ __global__ void __maxnreg__(kMarchRegs)
 
     RangeAcc racc;
     RingPos pm{0, 0};
-    for (int item = blockIdx.x; item < g.items; item += gridDim.x) {
-        const int ic = item / nJK;
-        const int jk = item - ic * nJK;
-        const int jb = jk / g.nKS;
-        const int k0s = (jk - jb * g.nKS) * KS;
-        const int j0 = jb * TJ, i0 = ic * g.CI;
-        const int ni = min(g.CI, n0 - i0);
-        const int jw = j0 + r - 1;
+    int run = 0, more = 1;
+    for (int item = blockIdx.x; BAL ? more : item < g.items; item += gridDim.x, ++run) {
         RingPos pc = pm, pp;
         pc.next(NS);
         pp = pc;
         pp.next(NS);
+        if (!mbar_wait(&full[pm.stage], pm.phase)) {
+            if (lane == 0) atomicExch(&g_device_status, (int)TIPT_ERR_TIMEOUT);
+            return;
+        }
+        int jk, i0, ni;
+        if constexpr (BAL) {
+            const int4 rs = *run_slot(full, run);
+            jk = rs.x;
+            i0 = rs.y;
+            ni = rs.z;
+            more = rs.w;
+        } else {
+            const int ic = item / nJK;
+            jk = item - ic * nJK;
+            i0 = ic * g.CI;
+            ni = min(g.CI, n0 - i0);
+        }
+        const int jb = jk / g.nKS;
+        const int k0s = (jk - jb * g.nKS) * KS;
+        const int jw = jb * TJ + r - 1;
         const int kcol = edge_l ? (k0s - 1 + n2) % n2 : (k0s + KS) % n2;
         if (edge) fetch_halo(i0, jw, kcol, 0);
-        if (!mbar_wait(&full[pm.stage], pm.phase) || !mbar_wait(&full[pc.stage], pc.phase)) {
+        if (!mbar_wait(&full[pc.stage], pc.phase)) {
             if (lane == 0) atomicExch(&g_device_status, (int)TIPT_ERR_TIMEOUT);
             if (edge) asm volatile("cp.async.wait_all;" ::: "memory");
             return;
@@ -1346,8 +1423,6 @@ static int g_force_tj = 0, g_force_ci = 0, g_force_stages = 0;
 // Kernels compiled for a fixed geometry used where the run-time geometry is
 // theirs (tipt_set_march_fixed(); on by default).
 static bool g_fixed_geom = true;
-// The compensated-FP32 stage's balanced split of the work (MarchGeom::bal).
-static bool g_balance = true;
 
 // One-shot test of the bounded waits (tipt_test_withhold_plane): the next
 // compensated-FP32 marching stage launch withholds a ring position in block 0.
@@ -1460,9 +1535,31 @@ bool march_supported(int storage, const RealStageParams& p) {
     return geometry(storage, p, tb, g, smem);
 }
 
+// How the work is split over `ctas` CTAs (MarchRuns), by the planes that the busiest
+// CTA computes: its items of CI planes, or an equal share of the (tile, plane) units.
+// Every run computes two planes' worth of prologue.  The equal shares put neighbouring
+// tiles at different planes, so a tile's halo rows are no longer in L2 from the
+// neighbour's reads: 6 % slower at 512^3 compensated FP32 with seven items a CTA (1.011
+// -> 1.075 ms), and that much they must save.  They matter below about 300^3, where
+// 64-plane items leave most SMs idle: 128^3 FP64 256 -> 36 us, 128^3 complex
+// compensated FP32 250 -> 53 us, 64^3 BAOAB 215 -> 32 us.
+static void split_work(MarchGeom& g, int tiles, int planes, int ctas, int loss) {
+    const int64_t units = (int64_t)tiles * planes;
+    const int64_t items = (int64_t)tiles * ((planes + g.CI - 1) / g.CI);
+    const int64_t rr = (items + ctas - 1) / ctas * ((g.CI < planes ? g.CI : planes) + 2);
+    const int64_t share = (units + ctas - 1) / ctas;
+    const int64_t eq = share + 2 * (1 + (share + planes - 2) / planes);
+    g.bal = eq * (100 + loss) < rr * 100 && units < 0x7FFFFFFF;
+    g.items = (int)(g.bal ? units : items);
+}
+
+// A batched ensemble's launch: its items run over the replicas.
+static bool has_replicas(const EnsMarch& em) { return em.reps != nullptr; }
+
 template <typename Kern, typename... Extra>
-static int launch_march_k(Kern kern, const RealStageParams& p, const MarchGeom& g, int64_t smem,
+static int launch_march_k(Kern kern, const RealStageParams& p, const MarchGeom& g_in, int64_t smem,
                           cudaStream_t st, Extra... extra) {
+    MarchGeom g = g_in;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e == cudaSuccess)
@@ -1476,6 +1573,7 @@ static int launch_march_k(Kern kern, const RealStageParams& p, const MarchGeom& 
         return fail(TIPT_ERR_UNSUPPORTED, "marching kernel does not fit an SM (%d threads, %lld "
                     "bytes of shared memory)", threads, (long long)smem);
     int grid = num_sms() * per_sm;
+    if (!(has_replicas(extra) || ...)) split_work(g, g.nJB, p.i_end - p.i_begin, grid, 40 / g.TJ);
     if (grid > g.items) grid = g.items;
     kern<<<grid, threads, (size_t)smem, st>>>(p, g, extra...);
     e = cudaGetLastError();
@@ -1563,27 +1661,13 @@ static int launch_f32c_stage(const RealStageParams& q, const MarchGeom& g0, int6
                              int64_t smem_table, cudaStream_t st) {
     const bool tab = q.table_in_smem && (q.vkind == TIPT_VP_TABLE || q.vkind == TIPT_VP_TABLE2D) &&
                      !q.noise;
-    // lattices with fewer CI-plane items than SMs: every CTA an equal share of the
-    // (j-block, plane) units, so every SM works.  (With more items the round-robin
-    // items stay: they keep the CTAs of neighbouring j-blocks at the same planes,
-    // so a tile's halo rows are still in L2 from the neighbour's reads; the
-    // j-block-major shares lose that reuse and measured 6 % slower at 512^3.)
-    const auto balance = [&](MarchGeom& b) {
-        if (!g_balance || b.items >= num_sms()) return;
-        b.bal = 1;
-        const int64_t units = (int64_t)b.nJB * (q.i_end - q.i_begin);
-        b.items = units < 0x7FFFFFFF ? (int)units : 0x7FFFFFFF;
-    };
     // the TAB kernels stage the row as (value, slope) pairs: twice the table bytes
     MarchGeom g;
     int64_t smem;
     if (!tab || !geometry(TIPT_F32C, q, 2 * smem_table, g, smem)) {
-        MarchGeom b = g0;
-        balance(b);
-        return launch_march_k(rk2_stage_march_f32c<WIDE, false, RG, false>, q, b, smem0, st,
+        return launch_march_k(rk2_stage_march_f32c<WIDE, false, RG, false>, q, g0, smem0, st,
                               EnsMarch{});
     }
-    balance(g);
     const bool exact = g_fixed_geom && g.pitch == q.n2 &&
                        g.stage_bytes == 4 * (g.TJ + 2) * g.pitch * 4;
     if (exact && q.n2 == 512 && g.TJ == 4)
@@ -1693,6 +1777,7 @@ static int launch_alt_march_k(const AltParams& p, cudaStream_t st) {
     if (e != cudaSuccess || per_sm < 1)
         return fail(TIPT_ERR_UNSUPPORTED, "integrator march kernel does not fit an SM");
     int grid = num_sms() * per_sm;
+    split_work(g, g.nJB, p.n0, grid, 40 / g.TJ);
     if (grid > g.items) grid = g.items;
     kern<<<grid, threads, (size_t)smem, st>>>(p, g);
     e = cudaGetLastError();
@@ -1809,26 +1894,26 @@ int launch_complex_march(const ComplexStageParams& p, cudaStream_t st) {
     // compiled with that geometry fixed
     const bool fixed = g_fixed_geom && g.KS == 256 && g.TJ == 4 && g.pitch == 256 &&
                        g.halo_off == 8 * 6 * 256 * 4 && g.stage_bytes == g.halo_off;
-    auto kern = fixed ? (p.range ? (wide ? complex_stage_march_f32c<true, true, 256, 4>
-                                         : complex_stage_march_f32c<false, true, 256, 4>)
-                                 : (wide ? complex_stage_march_f32c<true, false, 256, 4>
-                                         : complex_stage_march_f32c<false, false, 256, 4>))
-            : p.range ? (wide ? complex_stage_march_f32c<true, true> : complex_stage_march_f32c<false, true>)
-                      : (wide ? complex_stage_march_f32c<true, false> : complex_stage_march_f32c<false, false>);
+    const int threads = g.TJ * (g.KS / 2) + 32;
+    int grid = num_sms() * ctas_per_sm(g, g.KS / 2);
+    split_work(g, g.nJB * g.nKS, p.n0, grid, 100 / g.TJ);
+    if (grid > g.items) grid = g.items;
+    const auto pick = [&](auto bal) {
+        constexpr bool B = decltype(bal)::value;
+        return fixed ? (p.range ? (wide ? complex_stage_march_f32c<true, true, B, 256, 4>
+                                        : complex_stage_march_f32c<false, true, B, 256, 4>)
+                                : (wide ? complex_stage_march_f32c<true, false, B, 256, 4>
+                                        : complex_stage_march_f32c<false, false, B, 256, 4>))
+               : p.range ? (wide ? complex_stage_march_f32c<true, true, B> : complex_stage_march_f32c<false, true, B>)
+                         : (wide ? complex_stage_march_f32c<true, false, B> : complex_stage_march_f32c<false, false, B>);
+    };
+    auto kern = g.bal ? pick(std::true_type{}) : pick(std::false_type{});
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return fail_cuda(e, "complex marching kernel attributes");
-    const int threads = g.TJ * (g.KS / 2) + 32;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, (size_t)smem);
-    if (e != cudaSuccess || per_sm < 1)
-        return fail(TIPT_ERR_UNSUPPORTED, "complex marching kernel does not fit an SM (%d "
-                    "threads, %lld bytes of shared memory)", threads, (long long)smem);
-    int grid = num_sms() * per_sm;
-    if (grid > g.items) grid = g.items;
     kern<<<grid, threads, (size_t)smem, st>>>(tm[0], tm[1], tm[2], tm[3], p, g);
     e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "complex marching kernel launch");
