@@ -1,7 +1,7 @@
 """The marching kernels' equal shares of the work against the generic kernel, bit for bit, at
 shapes where a CTA's share is less than a plane run, spans several tiles, or ends inside one;
-beside them shapes that keep the round-robin items.  Every storage, both fields and the
-integrators."""
+beside them shapes that keep the round-robin items.  Every storage, the thermal source, both
+fields and the integrators."""
 import numpy as np
 import pytest
 
@@ -59,6 +59,18 @@ def test_real_step(shape, storage):
         for n in range(2):
             RF.rk2_step_table(*f, 0.05, 1.0, 1.0, 1.0, None, *t, 1.0, *table(), noise_scale=0.3,
                               noise_step=n, seed=2)
+        return f
+    both(run)
+
+
+@pytest.mark.parametrize("shape", SHAPES[:6])
+@pytest.mark.parametrize("storage", ["f64", "f32", "f32c"])
+def test_real_thermal(shape, storage):
+    def run():
+        f = state(shape, storage, 2)
+        t = [torch.empty_like(x) for x in f]
+        RF.rk2_fused_single_pass(*f, 0.05, 1.0, 1.0, 7350.0, 7349.0, 1000.0, 1e-24, 1000.0, 1e6,
+                                 1.09, 1.05, 1.09, 1.05, 0.3, 4, *t, 1.0)
         return f
     both(run)
 

@@ -133,6 +133,23 @@ __device__ __forceinline__ void sqrt_parts(double v, double& s, double& d) {
     d = __dmul_rn(__fma_rn(-s, s, v), h);
 }
 
+// y = 1/sqrt(v) and, with SQ, s = sqrt(v), both to about half an ulp, for v in
+// [1e-300, 1e300]: the hardware approximation and one step of third order
+// (Householder), (1 - e)^(-1/2) = 1 + e (1/2 + 3 e / 8) with e = 1 - v y0^2 from the
+// exact product v y0 = m + l.  Replaces a square root and the divisions by it: 7 to 9
+// FP64 operations and no branch.
+template <bool SQ>
+__device__ __forceinline__ void rsqrt_sqrt(double v, double& y, double& s) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(v));
+    const double m = __dmul_rn(v, y0);
+    const double l = __fma_rn(v, y0, -m);
+    const double e = __fma_rn(-l, y0, __fma_rn(-m, y0, 1.0));
+    const double w = __dmul_rn(e, __fma_rn(0.375, e, 0.5));
+    y = __fma_rn(y0, w, y0);
+    if constexpr (SQ) s = __dadd_rn(m, __fma_rn(m, w, l));
+}
+
 // sin y, |y| <= pi/2
 __device__ __forceinline__ double sin_half_pi(double y) {
     const double t = __dmul_rn(y, y);

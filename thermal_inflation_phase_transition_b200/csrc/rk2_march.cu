@@ -193,16 +193,6 @@ __device__ __forceinline__ void ld_pair_g(const E* p, E& a, E& b) {
     }
 }
 
-template <int S>
-__device__ __forceinline__ void site_update(const RealStageParams& p, const void* s_tab,
-                                            float, float, const typename MarchElem<S>::E ph[7],
-                                            const typename MarchElem<S>::E pv[7], double noise,
-                                            typename MarchElem<S>::E& a,
-                                            typename MarchElem<S>::E& b) {
-    if constexpr (S == TIPT_F64) update_f64(p, static_cast<const double*>(s_tab), ph, pv, noise, a, b);
-    else update_f32(p, static_cast<const double*>(s_tab), ph, pv, noise, a, b);
-}
-
 // Launch bounds of the two block-size classes: up to 256 consumer threads
 // (two CTAs per SM) or up to 512 (one CTA per SM), plus the producer warp.
 // Ring position -> (stage, phase parity), advanced incrementally.
@@ -267,11 +257,15 @@ __device__ __forceinline__ int4* run_slot(uint64_t* full, int run) {
     return reinterpret_cast<int4*>(full + 6 + 8 * (run & 1));
 }
 
-template <int S, bool WIDE>
+// TH: the thermal V' source; RG: the range of the new phi (RealStageParams::range).
+// float32: a thread keeps the midpoint values of its own four sites of planes i - 1 and
+// i, so it forms four of the seven that a site's stencil takes.
+template <int S, bool WIDE, bool TH, bool RG>
 __global__ void __maxnreg__(kMarchRegs)
     rk2_stage_march(RealStageParams p_in, MarchGeom g) {
     RealStageParams p = p_in;
     resolve_schedule(p);
+    if constexpr (RG) reset_next_range(p);
     using E = typename MarchElem<S>::E;
     using TT = typename MarchElem<S>::TT;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -360,11 +354,12 @@ __global__ void __maxnreg__(kMarchRegs)
     const int kpA = c + 2;                                    // right of pair A
     const int kmB = half + c - 1;                             // left of pair B
     const int kpB = half + c + 2 == n2 ? 0 : half + c + 2;    // right of pair B
-    const float tminf = (float)p.tmin, dinvf = (float)p.dinv;
+    const double* tab = static_cast<const double*>(s_tab);
     E* const phi_out = static_cast<E*>(p.phi_out);
     E* const pi_out = static_cast<E*>(p.pi_out);
     const int orow = r * pitch, urow = (r - 1) * pitch, drow = (r + 1) * pitch;
 
+    RangeAcc racc;
     RingPos pm{0, 0};  // ring position of plane i-1 for the current iteration
     for (int run = 0, more = 1; more; ++run) {
         RingPos pc = pm, pp;
@@ -378,6 +373,22 @@ __global__ void __maxnreg__(kMarchRegs)
         const int4 rs = *run_slot(full, run);
         const int jw = rs.x + r - 1, i0 = rs.y, ni = rs.z;
         more = rs.w;
+        float2 tm[2], tc[2];   // float32: phi~ of the own pairs in planes i - 1 and i
+        if constexpr (S == TIPT_F32) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int o = orow + (h ? half + c : c);
+                const auto pair = [&](uint32_t st, int f) {
+                    return *reinterpret_cast<const float2*>(fld(st, f) + o);
+                };
+                const auto mid = [&](uint32_t st) {
+                    const float2 a = pair(st, 0), v = pair(st, 1);
+                    return make_float2(midpoint_f32(p, a.x, v.x), midpoint_f32(p, a.y, v.y));
+                };
+                tm[h] = mid(pm.stage);
+                tc[h] = mid(pc.stage);
+            }
+        }
         for (int q = 0; q < ni; ++q) {
             const int i = i0 + q;
             const int64_t rowoff = ((int64_t)i * n1 + jw) * n2;
@@ -420,6 +431,17 @@ __global__ void __maxnreg__(kMarchRegs)
                     if (lane == 0) mbar_arrive(&empty[pm.stage]);
                 }
                 E op[2], ov[2];
+                float2 tp, tj, td, tk;
+                if constexpr (S == TIPT_F32) {
+                    const auto mid = [&](const float (&a)[2][2]) {
+                        return make_float2(midpoint_f32(p, a[0][0], a[1][0]),
+                                           midpoint_f32(p, a[0][1], a[1][1]));
+                    };
+                    tp = mid(ip);
+                    tj = mid(jp);
+                    td = mid(jm);
+                    tk = make_float2(midpoint_f32(p, kl[0], kl[1]), midpoint_f32(p, kr[0], kr[1]));
+                }
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     // stencil order: centre, ip, im, jp, jm, kp, km (R:1913-1920)
@@ -427,7 +449,21 @@ __global__ void __maxnreg__(kMarchRegs)
                                      u ? kr[0] : ce[0][1], u ? ce[0][0] : kl[0]};
                     const E pv[7] = {ce[1][u], ip[1][u], im[1][u], jp[1][u], jm[1][u],
                                      u ? kr[1] : ce[1][1], u ? ce[1][0] : kl[1]};
-                    site_update<S>(p, s_tab, tminf, dinvf, ph, pv, nz[h][u], op[u], ov[u]);
+                    if constexpr (S == TIPT_F64) {
+                        update_f64<TH>(p, tab, ph, pv, nz[h][u], op[u], ov[u]);
+                        if constexpr (RG) racc.fold_d(op[u]);
+                    } else {
+                        const float pt[7] = {u ? tc[h].y : tc[h].x, u ? tp.y : tp.x,
+                                             u ? tm[h].y : tm[h].x, u ? tj.y : tj.x,
+                                             u ? td.y : td.x,       u ? tk.y : tc[h].y,
+                                             u ? tc[h].x : tk.x};
+                        update_f32_mid<TH>(p, tab, ph, pt, pv[0], nz[h][u], op[u], ov[u]);
+                        if constexpr (RG) racc.fold(op[u]);
+                    }
+                }
+                if constexpr (S == TIPT_F32) {
+                    tm[h] = tc[h];
+                    tc[h] = tp;
                 }
                 st_pair_g(phi_out + rowoff + col, op[0], op[1]);
                 st_pair_g(pi_out + rowoff + col, ov[0], ov[1]);
@@ -442,8 +478,9 @@ __global__ void __maxnreg__(kMarchRegs)
             mbar_arrive(&empty[pm.stage]);
             mbar_arrive(&empty[pc.stage]);
         }
-        pm = pp;  // the next item starts at the following ring position
+        pm = pp;  // the next run starts at the following ring position
     }
+    if constexpr (RG) racc.flush(p.range);
 }
 
 // Batched-ensemble arguments of the compensated-FP32 marching stage (unused for
@@ -1524,7 +1561,6 @@ static bool geometry(int storage, const RealStageParams& p, int64_t smem_table, 
 
 bool march_supported(int storage, const RealStageParams& p) {
     if (storage != TIPT_F32C && storage != TIPT_F64 && storage != TIPT_F32) return false;
-    if (storage != TIPT_F32C && p.range) return false;  // the generic kernel folds the range
     const uintptr_t a = reinterpret_cast<uintptr_t>(p.phi) | reinterpret_cast<uintptr_t>(p.pi) |
                         reinterpret_cast<uintptr_t>(p.phi_out) |
                         reinterpret_cast<uintptr_t>(p.pi_out);
@@ -1680,6 +1716,21 @@ static int launch_f32c_stage(const RealStageParams& q, const MarchGeom& g0, int6
                           EnsMarch{});
 }
 
+// The FP64 and float32 storages' stage.
+template <int S>
+static int launch_fp64_stage(const RealStageParams& p, const MarchGeom& g, int64_t smem, bool wide,
+                             cudaStream_t st) {
+    const auto go = [&](auto th, auto rg) {
+        constexpr bool TH = decltype(th)::value, RG = decltype(rg)::value;
+        return wide ? launch_march_k(rk2_stage_march<S, true, TH, RG>, p, g, smem, st)
+                    : launch_march_k(rk2_stage_march<S, false, TH, RG>, p, g, smem, st);
+    };
+    constexpr std::true_type yes;
+    constexpr std::false_type no;
+    if (p.vkind == TIPT_VP_THERMAL) return p.range ? go(yes, yes) : go(yes, no);
+    return p.range ? go(no, yes) : go(no, no);
+}
+
 int launch_march(int storage, const RealStageParams& p, int64_t smem_table, cudaStream_t st) {
     MarchGeom g;
     int64_t smem;
@@ -1705,14 +1756,8 @@ int launch_march(int storage, const RealStageParams& p, int64_t smem_table, cuda
         return wide ? launch_f32c_stage<true, false>(q, g, smem, smem_table, st)
                     : launch_f32c_stage<false, false>(q, g, smem, smem_table, st);
     }
-    if (storage != TIPT_F32C && p.range)
-        return fail(TIPT_ERR_UNSUPPORTED, "the FP64 / float32 marching stage takes no range output");
-    if (storage == TIPT_F64)
-        return wide ? launch_march_k(rk2_stage_march<TIPT_F64, true>, p, g, smem, st)
-                    : launch_march_k(rk2_stage_march<TIPT_F64, false>, p, g, smem, st);
-    if (storage == TIPT_F32)
-        return wide ? launch_march_k(rk2_stage_march<TIPT_F32, true>, p, g, smem, st)
-                    : launch_march_k(rk2_stage_march<TIPT_F32, false>, p, g, smem, st);
+    if (storage == TIPT_F64) return launch_fp64_stage<TIPT_F64>(p, g, smem, wide, st);
+    if (storage == TIPT_F32) return launch_fp64_stage<TIPT_F32>(p, g, smem, wide, st);
     return fail(TIPT_ERR_STORAGE, "marching kernel takes F32C, F64 or F32");
 }
 

@@ -60,6 +60,20 @@ static void canonical_shape(RealStageParams& p) {
     }
 }
 
+// Whether the marching kernel is the faster one where it applies.  It runs 17 warps an
+// SM against the generic kernel's 32, so it hides latency worse:
+//  * the inline thermal V', long FP64 chains (256^3, two halves: FP64 1032 against 841 us,
+//    float32 1009 against 894 us), except in compensated FP32 on large lattices, whose
+//    stencil reads four components (256^3 804 against 853 us, 96^3 67 against 54 us);
+//  * a noise array in the FP64 and float32 storages, loaded where the hash would be
+//    drawn (the script's loop: 256^3 FP64 469 against 316 us, float32 344 against 337).
+// With hash noise it wins: 256^3 FP64 227 against 259 us, float32 227 against 279 us.
+static bool march_pays(int storage, const RealStageParams& p) {
+    if (p.vkind == TIPT_VP_THERMAL)
+        return storage == TIPT_F32C && (int64_t)p.n0 * p.n1 * p.n2 >= 6 << 20;
+    return storage == TIPT_F32C || !p.noise;
+}
+
 int launch_real_stage(int storage, RealStageParams p, cudaStream_t st) {
     if (p.i_end == 0) {
         canonical_shape(p);
@@ -73,7 +87,8 @@ int launch_real_stage(int storage, RealStageParams p, cudaStream_t st) {
                     "shared memory", p.npts, (long long)kMaxTableSmem);
     const int64_t smem = p.table_in_smem ? tb : 0;
     set_f32c_pairs(p);
-    const bool march = g_kernel_policy != 1 && march_supported(storage, p);
+    const bool march = g_kernel_policy != 1 && march_supported(storage, p) &&
+                       (g_kernel_policy == 2 || march_pays(storage, p));
     if (g_kernel_policy == 2 && !march)
         return fail(TIPT_ERR_UNSUPPORTED, "marching kernel does not cover this shape/storage");
     if (march) return launch_march(storage, p, smem, st);

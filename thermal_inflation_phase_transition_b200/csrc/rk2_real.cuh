@@ -101,6 +101,12 @@ __device__ __forceinline__ void resolve_schedule(RealStageParams& p) {
     p.step += s;
 }
 
+// A lane-pair constant as a lane vector.
+__device__ __forceinline__ float kv(float2 c, float) { return c.x; }
+__device__ __forceinline__ float2 kv(float2 c, float2) { return c; }
+template <typename V>
+__device__ __forceinline__ V kvec(float2 c) { return kv(c, V{}); }
+
 // Row-blend weight of a 2-D table (same trunc/clamp/unclamped-weight rule
 // along T as along phi).
 __device__ __forceinline__ void table2d_row(const RealStageParams& p, int& it, double& w) {
@@ -201,12 +207,6 @@ __host__ __device__ inline void set_f32c_pairs(RealStageParams& p) {
     p.k2.tmd = pr((float)(-p.tmin * p.dinv));
 }
 
-// A lane-pair constant as a lane vector.
-__device__ __forceinline__ float kv(float2 c, float) { return c.x; }
-__device__ __forceinline__ float2 kv(float2 c, float2) { return c; }
-template <typename V>
-__device__ __forceinline__ V kvec(float2 c) { return kv(c, V{}); }
-
 __device__ __forceinline__ F32CConst f32c_const(const RealStageParams& p) {
     F32CConst k;
     k.h1 = (float)p.h1;
@@ -292,27 +292,44 @@ __device__ __forceinline__ void update_f64(const RealStageParams& p, const doubl
 }
 
 // --------------------------------------------------------------- F32 ----
-// The reference's float32 mode (USE_FLOAT32, R:348): float32 neighbour sums, FP64
-// for the rest, float32 stores, among them the midpoint's pi~ (R:1933).  The
-// midpoint's phi~ stays in FP64: the reference rounds it to float32 at every
-// neighbour (R:1932), which here would be 27 conversions between FP32 and FP64 a
-// site (their unit bound the stage) for a less exact Laplacian.
+// The reference's float32 mode (USE_FLOAT32, R:348): float32 neighbour sums,
+// FP64 for the rest, float32 stores -- including the stored midpoint state
+// phi~, pi~ that pass 2 reads (R:1932-1933).
 __device__ __forceinline__ float sum6_f(const float v[7]) {
     return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(v[1], v[2]), v[3]), v[4]), v[5]), v[6]);
+}
+
+// phi~ = phi + h1 pi in FP64, rounded to float32.  Its rounding is kept as it is at every
+// neighbour: with h1 a round decimal phi~ lies within 1e-9 ulp of a tie at one site in
+// 5000, so other routes to the same value (a Laplacian linear in phi and pi, float pairs)
+// change that many last bits, which observables summed in FP64 show.
+template <class P>
+__device__ __forceinline__ float midpoint_f32(const P& p, float ph, float pv) {
+    return __double2float_rn(__fma_rn(p.h1, (double)pv, (double)ph));
+}
+
+// The update from the stencils of phi and phi~.
+template <bool TH = true>
+__device__ __forceinline__ void update_f32_mid(const RealStageParams& p, const double* s_tab,
+                                               const float ph[7], const float pt[7], float pv,
+                                               double noise, float& phi_new, float& pi_new) {
+    const double c = (double)ph[0], ct = (double)pt[0], v = (double)pv;
+    const double lap = __dmul_rn(__fma_rn(-6.0, c, (double)sum6_f(ph)), p.inv_dx2);
+    const double lap2 = __dmul_rn(__fma_rn(-6.0, ct, (double)sum6_f(pt)), p.inv_dx2);
+    const double k1 = force_d(p, lap, v, vprime_d<TH>(p, s_tab, c));
+    const double pit = (double)__double2float_rn(__fma_rn(p.h1, k1, v));
+    const double k2 = force_d(p, lap2, pit, vprime_d<TH>(p, s_tab, ct));
+    phi_new = __double2float_rn(__fma_rn(p.h2, pit, c));
+    pi_new = __double2float_rn(__dadd_rn(v, __fma_rn(p.h2, k2, noise)));
 }
 template <bool TH = true>
 __device__ __forceinline__ void update_f32(const RealStageParams& p, const double* s_tab,
                                            const float ph[7], const float pv[7], double noise,
                                            float& phi_new, float& pi_new) {
-    const double c = (double)ph[0], v = (double)pv[0];
-    const double lap = __dmul_rn(__fma_rn(-6.0, c, (double)sum6_f(ph)), p.inv_dx2);
-    const double lapv = __dmul_rn(__fma_rn(-6.0, v, (double)sum6_f(pv)), p.inv_dx2);
-    const double k1 = force_d(p, lap, v, vprime_d<TH>(p, s_tab, c));
-    const double pit = (double)__double2float_rn(__fma_rn(p.h1, k1, v));
-    const double k2 = force_d(p, __fma_rn(p.h1, lapv, lap), pit,
-                              vprime_d<TH>(p, s_tab, __fma_rn(p.h1, v, c)));
-    phi_new = __double2float_rn(__fma_rn(p.h2, pit, c));
-    pi_new = __double2float_rn(__dadd_rn(v, __fma_rn(p.h2, k2, noise)));
+    float pt[7];
+#pragma unroll
+    for (int q = 0; q < 7; ++q) pt[q] = midpoint_f32(p, ph[q], pv[q]);
+    update_f32_mid<TH>(p, s_tab, ph, pt, pv[0], noise, phi_new, pi_new);
 }
 
 // -------------------------------------------------------------- F32C ----

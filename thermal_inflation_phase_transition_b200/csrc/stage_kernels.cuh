@@ -35,12 +35,12 @@ struct FastDiv {
 
 // One site per thread (grid stride): the stencil straight from global memory through
 // L1.  Bound: the latency of the loads and of the FP64 chains (64 registers a thread,
-// four blocks an SM; five or six blocks spill), then issue.  Coordinates by two
-// multiplications and 32-bit site indices instead of 64-bit divisions and addresses,
-// and no midpoint value per neighbour (rk2_real.cuh): a 256^3 float32 stage with
-// noise array, 16384-point table and range 283 -> 163 us (298 -> 189 instructions a
-// site), the complex one at 512x512x64 534 -> 370 us.  (A tile walking the planes
-// with the midpoint field in shared memory measured 251 us, and slower on odd rows.)
+// four blocks an SM; five or six blocks spill), then issue and, in float32 storage, the
+// conversions.  Coordinates by two multiplications and 32-bit site indices instead of
+// 64-bit divisions and addresses: a 256^3 float32 stage with noise array, 16384-point
+// table and range 283 -> 210 us, the complex one at 512x512x64 534 -> 420 us.  (A tile
+// walking the planes with the midpoint field in shared memory measured 251 us, and
+// slower on odd rows.)
 struct GenericGeom {
     FastDiv d1, d2;
     int i_begin, i_end;

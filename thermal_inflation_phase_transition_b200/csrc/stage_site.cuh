@@ -161,7 +161,7 @@ struct ComplexSite {
                         q2d = (double)nb[2][0] + ((double)nb[3][0] + (double)h1 * ((double)nb[6][0] + (double)nb[7][0]));
                     }
                     double e1, e2;
-                    complex_force<double, TH>(p, p.table, p.tmin, p.dinv, q1d, q2d, e1, e2);
+                    complex_force<TH>(p, p.table, q1d, q2d, e1, e2);
                     d1 = (float)e1;
                     d2 = (float)e2;
                 }
@@ -183,30 +183,43 @@ struct ComplexSite {
             }
             if constexpr (RG) fold_rho_ff(racc, oh[0], ol[0], oh[1], ol[1]);
         } else {
-            // FP64 arithmetic after the neighbour sums; float32 storage sums neighbours and
-            // stores the midpoint's pi in float32 (as update_f32).  The Laplacian of
-            // phi + h1 pi is lap + h1 lap(pi).
+            // FP64 arithmetic after the neighbour sums.  The Laplacian of phi~ = phi + h1 pi
+            // is lap + h1 lap(pi); float32 storage takes it from the float32 phi~ and rounds
+            // the midpoint's pi, as the reference stores them (see update_f32).
             const double* tab = p.table_in_smem ? static_cast<const double*>(s_tab) : p.table;
-            double c[4], lap[4];
+            const auto lap_of = [&](const E v[7], double c) {
+                const E s6 = v[1] + v[2] + v[3] + v[4] + v[5] + v[6];
+                return __dmul_rn(__fma_rn(-6.0, c, (double)s6), p.inv_dx2);
+            };
+            double c[4], lap[2], lapt[2], q[2];   // q: phi~ at the site
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const E s6 = nb[r][1] + nb[r][2] + nb[r][3] + nb[r][4] + nb[r][5] + nb[r][6];
-                c[r] = (double)nb[r][0];
-                lap[r] = ((double)s6 - 6.0 * c[r]) * p.inv_dx2;
+            for (int r = 0; r < 4; ++r) c[r] = (double)nb[r][0];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                lap[a] = lap_of(nb[a], c[a]);
+                if constexpr (S == TIPT_F32) {
+                    float pt[7];
+#pragma unroll
+                    for (int r = 0; r < 7; ++r) pt[r] = midpoint_f32(p, nb[a][r], nb[2 + a][r]);
+                    q[a] = (double)pt[0];
+                    lapt[a] = lap_of(pt, q[a]);
+                } else {
+                    q[a] = __fma_rn(p.h1, c[2 + a], c[a]);
+                    lapt[a] = __fma_rn(p.h1, lap_of(nb[2 + a], c[2 + a]), lap[a]);
+                }
             }
             double d[2], pt[2], n[2];
-            complex_force<double, TH>(p, tab, p.tmin, p.dinv, c[0], c[1], d[0], d[1]);
+            complex_force<TH>(p, tab, c[0], c[1], d[0], d[1]);
 #pragma unroll
             for (int a = 0; a < 2; ++a)
                 pt[a] = (double)(E)(c[2 + a] + p.h1 * (p.inv_a2 * lap[a] - p.eta * c[2 + a] -
                                                        d[a] * p.inv_mu2));
-            complex_force<double, TH>(p, tab, p.tmin, p.dinv, c[0] + p.h1 * c[2], c[1] + p.h1 * c[3],
-                                      d[0], d[1]);
+            complex_force<TH>(p, tab, q[0], q[1], d[0], d[1]);
             complex_noise<E>(p, (uint64_t)s, n[0], n[1]);
             E o[2];
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
-                const double k2 = p.inv_a2 * (lap[a] + p.h1 * lap[2 + a]) - p.eta * pt[a] - d[a] * p.inv_mu2;
+                const double k2 = p.inv_a2 * lapt[a] - p.eta * pt[a] - d[a] * p.inv_mu2;
                 o[a] = (E)(c[a] + p.h2 * pt[a]);
                 static_cast<E*>(p.o[a])[s] = o[a];
                 static_cast<E*>(p.o[2 + a])[s] = (E)(c[2 + a] + (p.h2 * k2 + n[a]));
