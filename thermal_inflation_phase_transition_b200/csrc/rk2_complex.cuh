@@ -23,6 +23,7 @@ struct ComplexStageParams {
     void* o[4];
     int n0, n1, n2;
     double h1, h2, inv_dx2, eta, inv_mu2, inv_a2;
+    double h1s;         // h1 2^896 (midpoint_f32_bits)
     const void* noise1;
     const void* noise2;
     double ns_eff, nfac;
@@ -47,6 +48,7 @@ struct ComplexStageParams {
 __host__ __device__ inline void set_complex_f32(ComplexStageParams& p) {
     auto pr = [](float x) { return make_float2(x, x); };
     const float h2h = (float)p.h2;
+    p.h1s = p.h1 * 0x1p896;
     p.k2.h1 = pr((float)p.h1);
     p.k2.h2h = pr(h2h);
     p.k2.h2l = pr((float)(p.h2 - (double)h2h));

@@ -21,6 +21,7 @@ struct RealStageParams {
     void* pi_out;
     int n0, n1, n2;      // lattice extents (nx, ny, nz); n2 contiguous
     double h1, h2;       // midpoint offset, advance
+    double h1s;          // h1 2^896 (midpoint_f32_bits)
     double inv_dx2, eta, inv_mu2, inv_a2;
     const void* noise;   // array noise (storage precision) or nullptr
     double ns_eff;       // hash noise amplitude incl. the 1/2 of half steps
@@ -189,6 +190,7 @@ struct F32CConst {
 __host__ __device__ inline void set_f32c_pairs(RealStageParams& p) {
     auto pr = [](float x) { return make_float2(x, x); };
     const float h2h = (float)p.h2;
+    p.h1s = p.h1 * 0x1p896;
     p.k2.h1 = pr((float)p.h1);
     p.k2.h2h = pr(h2h);
     p.k2.h2l = pr((float)(p.h2 - (double)h2h));
@@ -306,6 +308,19 @@ __device__ __forceinline__ float sum6_f(const float v[7]) {
 template <class P>
 __device__ __forceinline__ float midpoint_f32(const P& p, float ph, float pv) {
     return __double2float_rn(__fma_rn(p.h1, (double)pv, (double)ph));
+}
+// The same value, pi brought to FP64 by its bits: a float's sign, exponent and mantissa
+// fields as a double are the float times 2^-896, exactly, zeros and denormals included,
+// and h1s = h1 2^896 takes the factor.  For the kernels that the conversion unit bounds
+// (one warp instruction in eight cycles): the float32 script loops 313 -> 303 us (real,
+// 256^3) and 607 -> 583 us (complex, 512x512x64); the thermal stages lose 1 %.  (An
+// infinity becomes 2^128, which rounds to one again; a NaN is lost here, but phi's own
+// stencil carries it into every output.)
+template <class P>
+__device__ __forceinline__ float midpoint_f32_bits(const P& p, float ph, float pv) {
+    const int b = __float_as_int(pv);
+    const double s = __hiloint2double((b >> 3) & (int)0x8FFFFFFF, b << 29);
+    return __double2float_rn(__fma_rn(p.h1s, s, (double)ph));
 }
 
 // The update from the stencils of phi and phi~.

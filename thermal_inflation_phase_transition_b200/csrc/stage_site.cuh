@@ -1,8 +1,8 @@
 // What a midpoint stage does at one site, for the real and the complex field in
-// every storage: the values it reads at a site, and the update from the seven stencil
-// values of each.
+// every storage: what it reads at a site (load), the values its stencil takes there
+// (values) and the update from the seven stencil values of each.
 //
-// Stencil order of nb[r]: centre, ip, im, jp, jm, kp, km (R:1913-1920).
+// Stencil order of nb[v]: centre, ip, im, jp, jm, kp, km (R:1913-1920).
 #pragma once
 
 #include <type_traits>
@@ -37,6 +37,7 @@ struct RealSite {
     static constexpr int S = S_;
     static constexpr bool RG = RG_;
     static constexpr int NR = S == TIPT_F32C ? 4 : 2;  // phi, pi; with F32C each hi, lo
+    static constexpr int NV = S == TIPT_F32 ? 3 : NR;  // as read; float32: phi, phi~, pi
 
     static __device__ __forceinline__ void prepare(Params& p) {
         resolve_schedule(p);
@@ -59,8 +60,18 @@ struct RealSite {
             raw[1] = __ldg(pi + s);
         }
     }
+    static __device__ __forceinline__ void values(const Params& p, const E raw[NR], E v[NV]) {
+        if constexpr (S == TIPT_F32) {
+            v[0] = raw[0];
+            v[1] = TH ? midpoint_f32(p, raw[0], raw[1]) : midpoint_f32_bits(p, raw[0], raw[1]);
+            v[2] = raw[1];
+        } else {
+#pragma unroll
+            for (int q = 0; q < NV; ++q) v[q] = raw[q];
+        }
+    }
     static __device__ __forceinline__ void update(const Params& p, const F32CConst& kc,
-                                                  const void* s_tab, const E nb[NR][7],
+                                                  const void* s_tab, const E nb[NV][7],
                                                   int64_t s, int64_t N, RangeAcc& racc) {
         const uint64_t site = (uint64_t)(s + p.site_offset);
         E* po = static_cast<E*>(p.phi_out);
@@ -90,7 +101,7 @@ struct RealSite {
                 update_f64<TH>(p, tab, nb[0], nb[1], noise, a, b);
                 if constexpr (RG) racc.fold_d(a);
             } else {
-                update_f32<TH>(p, tab, nb[0], nb[1], noise, a, b);
+                update_f32_mid<TH>(p, tab, nb[0], nb[1], nb[2][0], noise, a, b);
                 if constexpr (RG) racc.fold(a);
             }
             po[s] = a;
@@ -108,6 +119,7 @@ struct ComplexSite {
     static constexpr int S = S_;
     static constexpr bool RG = RG_;
     static constexpr int NR = S == TIPT_F32C ? 8 : 4;  // phi1, phi2, pi1, pi2; F32C: hi, lo each
+    static constexpr int NV = S == TIPT_F32 ? 6 : NR;  // as read; float32: phi, phi~, pi
 
     static __device__ __forceinline__ void prepare(Params& p) {
         if constexpr (RG) reset_range_words(p.range_next);
@@ -130,8 +142,22 @@ struct ComplexSite {
             }
         }
     }
+    static __device__ __forceinline__ void values(const Params& p, const E raw[NR], E v[NV]) {
+        if constexpr (S == TIPT_F32) {
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                v[a] = raw[a];
+                v[2 + a] = TH ? midpoint_f32(p, raw[a], raw[2 + a])
+                              : midpoint_f32_bits(p, raw[a], raw[2 + a]);
+                v[4 + a] = raw[2 + a];
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < NV; ++q) v[q] = raw[q];
+        }
+    }
     static __device__ __forceinline__ void update(const Params& p, const F32CConst&,
-                                                  const void* s_tab, const E nb[NR][7],
+                                                  const void* s_tab, const E nb[NV][7],
                                                   int64_t s, int64_t N, RangeAcc& racc) {
         if constexpr (S == TIPT_F32C) {
             // planar {hi, lo} fields; FP32 forces, float-float state updates
@@ -191,18 +217,16 @@ struct ComplexSite {
                 const E s6 = v[1] + v[2] + v[3] + v[4] + v[5] + v[6];
                 return __dmul_rn(__fma_rn(-6.0, c, (double)s6), p.inv_dx2);
             };
-            double c[4], lap[2], lapt[2], q[2];   // q: phi~ at the site
-#pragma unroll
-            for (int r = 0; r < 4; ++r) c[r] = (double)nb[r][0];
+            constexpr int PI = S == TIPT_F32 ? 4 : 2;   // pi1 among the values
+            double c[4], lap[2], lapt[2], q[2];         // q: phi~ at the site
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
+                c[a] = (double)nb[a][0];
+                c[2 + a] = (double)nb[PI + a][0];
                 lap[a] = lap_of(nb[a], c[a]);
                 if constexpr (S == TIPT_F32) {
-                    float pt[7];
-#pragma unroll
-                    for (int r = 0; r < 7; ++r) pt[r] = midpoint_f32(p, nb[a][r], nb[2 + a][r]);
-                    q[a] = (double)pt[0];
-                    lapt[a] = lap_of(pt, q[a]);
+                    q[a] = (double)nb[2 + a][0];
+                    lapt[a] = lap_of(nb[2 + a], q[a]);
                 } else {
                     q[a] = __fma_rn(p.h1, c[2 + a], c[a]);
                     lapt[a] = __fma_rn(p.h1, lap_of(nb[2 + a], c[2 + a]), lap[a]);
