@@ -21,6 +21,7 @@
 // float-float state updates).
 #include <cstring>
 
+#include "column_walk.cuh"
 #include "integrators.cuh"
 #include "rk2_march.cuh"
 #include "tipt_internal.h"
@@ -60,39 +61,42 @@ __device__ __forceinline__ const TT* stage_alt_table(const AltParams& p, TT* s_t
     return s_tab;
 }
 
+// Any lattice shape on the column walk (column_walk.cuh); a table goes to shared memory once
+// per resident block.  Bound by the latency of the loads and of the force and noise chains.
+// Resident blocks per SM, measured at 3 / 4 / 5 / 6 (us): complex float32 256^3 overdamped
+// 239 / 245 / 255 / 257 (one site per thread with 64-bit divisions and seven reads: 281),
+// complex F32C 131x133x127 BAOAB 146 / 175 / 184 / 185 (193), complex FP64 192x190x188 BAOAB
+// 302 / 252 / 295 / 255 (289), real FP64 256^3 BAOAB 423 / 337 / 305 / 287 (417), real float32
+// 256^3 overdamped 169 / 166 / 165 / 166 (251).
+template <int S, bool CPLX>
+constexpr int alt_blocks() {
+    return CPLX ? (S == TIPT_F64 ? 4 : 3) : 6;
+}
+
 // ----------------------------------------------------------------- real ----
-template <int S, int MODE>
-__global__ void __launch_bounds__(256) alt_real_kernel(AltParams p) {
+template <int S, int MODE, typename I>
+__global__ void __launch_bounds__(256, (alt_blocks<S, false>())) alt_real_kernel(AltParams p, ColumnGeom g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using TT = typename std::conditional<S == TIPT_F32C, float, double>::type;
     const TT* s_tab = stage_alt_table<TT>(p, reinterpret_cast<TT*>(smem_raw));
     const double* dtab = p.v.table_in_smem ? reinterpret_cast<const double*>(s_tab) : p.v.table;
-    const int64_t n12 = (int64_t)p.n1 * p.n2;
-    const int64_t N = (int64_t)p.n0 * n12;
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int k = (int)(s % p.n2);
-        const int64_t r = s / p.n2;
-        const int j = (int)(r % p.n1);
-        const int i = (int)(r / p.n1);
-        const int64_t idx[7] = {
-            s, s + ((i + 1 < p.n0) ? n12 : -(int64_t)(p.n0 - 1) * n12),
-            s + ((i > 0) ? -n12 : (int64_t)(p.n0 - 1) * n12),
-            s + ((j + 1 < p.n1) ? (int64_t)p.n2 : -(int64_t)(p.n1 - 1) * p.n2),
-            s + ((j > 0) ? -(int64_t)p.n2 : (int64_t)(p.n1 - 1) * p.n2),
-            s + ((k + 1 < p.n2) ? 1 : -(int64_t)(p.n2 - 1)), s + ((k > 0) ? -1 : (int64_t)(p.n2 - 1))};
-        const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
+    const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
+    const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
+    // the stored planes of a site: phi, or its hi and lo parts
+    using E = typename std::conditional<S == TIPT_F64, double, float>::type;
+    constexpr int NV = S == TIPT_F32C ? 2 : 1;
+    const E* phi = static_cast<const E*>(p.f[0]);
+    const auto value = [&](int64_t s, E (&v)[NV]) {
+        v[0] = __ldg(phi + s);
+        if constexpr (S == TIPT_F32C) v[1] = __ldg(phi + N + s);
+    };
+    walk_columns<E, NV, I>(g, value, [&](int64_t s, const E (&nb)[NV][7]) {
         const uint64_t key = noise_key((uint64_t)s, p.step, kPass2Mul, p.seed);
         if constexpr (S == TIPT_F64 || S == TIPT_F32) {
-            using E = typename std::conditional<S == TIPT_F64, double, float>::type;
-            const E* phi = static_cast<const E*>(p.f[0]);
-            E q[7];
-#pragma unroll
-            for (int n = 0; n < 7; ++n) q[n] = __ldg(phi + idx[n]);
             double lap;
-            if constexpr (S == TIPT_F64) lap = lap_d(q, p.inv_dx2);
-            else lap = lap_f(q, p.inv_dx2);
-            const double ph = (double)q[0];
+            if constexpr (S == TIPT_F64) lap = lap_d(nb[0], p.inv_dx2);
+            else lap = lap_f(nb[0], p.inv_dx2);
+            const double ph = (double)nb[0][0];
             const double F = force_d(p, lap, vprime_alt_d(p.v, dtab, ph));
             const double z = noisy ? gauss_cos(key) : 0.0;
             if constexpr (MODE == kOD) {
@@ -111,16 +115,9 @@ __global__ void __launch_bounds__(256) alt_real_kernel(AltParams p) {
                 }
             }
         } else {
-            const float* phi = static_cast<const float*>(p.f[0]);
-            float hh[7], hl[7];
-#pragma unroll
-            for (int n = 0; n < 7; ++n) {
-                hh[n] = __ldg(phi + idx[n]);
-                hl[n] = __ldg(phi + N + idx[n]);
-            }
             float dh, dl;
-            stencil_sums(hh, hl, dh, dl);
-            const float vp = vprime_alt_f(p.v, s_tab, __fadd_rn(hh[0], hl[0]));
+            stencil_sums(nb[0], nb[1], dh, dl);
+            const float vp = vprime_alt_f(p.v, s_tab, __fadd_rn(nb[0][0], nb[1][0]));
             const float z = noisy ? gauss_cos_f(key) : 0.0f;
             float* out0 = static_cast<float*>(p.o[0]);
             float* out1 = static_cast<float*>(p.o[1]);
@@ -130,7 +127,7 @@ __global__ void __launch_bounds__(256) alt_real_kernel(AltParams p) {
                 vh = pif[s];
                 vl = pif[N + s];
             }
-            alt_real_site_f32c<MODE>(p, hh[0], hl[0], dh, dl, vp, z, vh, vl, ah, al, bh, bl);
+            alt_real_site_f32c<MODE>(p, nb[0][0], nb[1][0], dh, dl, vp, z, vh, vl, ah, al, bh, bl);
             if constexpr (MODE != kBA2) {
                 out0[s] = ah;
                 out0[N + s] = al;
@@ -140,45 +137,39 @@ __global__ void __launch_bounds__(256) alt_real_kernel(AltParams p) {
                 out1[N + s] = bl;
             }
         }
-    }
+    });
 }
 
 // -------------------------------------------------------------- complex ----
-template <int S, int MODE>
-__global__ void __launch_bounds__(256) alt_complex_kernel(AltParams p) {
+template <int S, int MODE, typename I>
+__global__ void __launch_bounds__(256, (alt_blocks<S, true>())) alt_complex_kernel(AltParams p, ColumnGeom g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using TT = typename std::conditional<S == TIPT_F32C, float, double>::type;
     const TT* s_tab = stage_alt_table<TT>(p, reinterpret_cast<TT*>(smem_raw));
     const double* dtab = p.v.table_in_smem ? reinterpret_cast<const double*>(s_tab) : p.v.table;
     const bool zn = p.v.zn_active > 0.5 && p.v.zn_n > 0.5;
-    const int64_t n12 = (int64_t)p.n1 * p.n2;
-    const int64_t N = (int64_t)p.n0 * n12;
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int k = (int)(s % p.n2);
-        const int64_t r = s / p.n2;
-        const int j = (int)(r % p.n1);
-        const int i = (int)(r / p.n1);
-        const int64_t idx[7] = {
-            s, s + ((i + 1 < p.n0) ? n12 : -(int64_t)(p.n0 - 1) * n12),
-            s + ((i > 0) ? -n12 : (int64_t)(p.n0 - 1) * n12),
-            s + ((j + 1 < p.n1) ? (int64_t)p.n2 : -(int64_t)(p.n1 - 1) * p.n2),
-            s + ((j > 0) ? -(int64_t)p.n2 : (int64_t)(p.n1 - 1) * p.n2),
-            s + ((k + 1 < p.n2) ? 1 : -(int64_t)(p.n2 - 1)), s + ((k > 0) ? -1 : (int64_t)(p.n2 - 1))};
-        const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
+    const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
+    const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
+    // the stored planes of a site: phi1 and phi2, or their hi parts and their lo parts
+    using E = typename std::conditional<S == TIPT_F64, double, float>::type;
+    constexpr int NV = S == TIPT_F32C ? 4 : 2;
+    const auto value = [&](int64_t s, E (&v)[NV]) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            const E* ph = static_cast<const E*>(p.f[a]);
+            v[a] = __ldg(ph + s);
+            if constexpr (S == TIPT_F32C) v[2 + a] = __ldg(ph + N + s);
+        }
+    };
+    walk_columns<E, NV, I>(g, value, [&](int64_t s, const E (&nb)[NV][7]) {
         const uint64_t key = noise_key((uint64_t)s, p.step, kPass2Mul, p.seed);
         if constexpr (S == TIPT_F64 || S == TIPT_F32) {
-            using E = typename std::conditional<S == TIPT_F64, double, float>::type;
             double lap[2], c[2];
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
-                const E* ph = static_cast<const E*>(p.f[a]);
-                E q[7];
-#pragma unroll
-                for (int n = 0; n < 7; ++n) q[n] = __ldg(ph + idx[n]);
-                if constexpr (S == TIPT_F64) lap[a] = lap_d(q, p.inv_dx2);
-                else lap[a] = lap_f(q, p.inv_dx2);
-                c[a] = (double)q[0];
+                if constexpr (S == TIPT_F64) lap[a] = lap_d(nb[a], p.inv_dx2);
+                else lap[a] = lap_f(nb[a], p.inv_dx2);
+                c[a] = (double)nb[a][0];
             }
             double d1, d2;
             complex_force<false>(p.v, dtab, c[0], c[1], d1, d2);
@@ -208,18 +199,11 @@ __global__ void __launch_bounds__(256) alt_complex_kernel(AltParams p) {
             float ch[2], cl[2], lap[2];
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
-                const float* ph = static_cast<const float*>(p.f[a]);
-                float hh[7], hl[7];
-#pragma unroll
-                for (int n = 0; n < 7; ++n) {
-                    hh[n] = __ldg(ph + idx[n]);
-                    hl[n] = __ldg(ph + N + idx[n]);
-                }
                 float dh, dl;
-                stencil_sums(hh, hl, dh, dl);
+                stencil_sums(nb[a], nb[2 + a], dh, dl);
                 lap[a] = __fmul_rn(__fadd_rn(dh, dl), (float)p.inv_dx2);
-                ch[a] = hh[0];
-                cl[a] = hl[0];
+                ch[a] = nb[a][0];
+                cl[a] = nb[2 + a][0];
             }
             float d1, d2;
             if (!zn && (p.v.table_in_smem || p.v.vkind == TIPT_VP_POLY)) {
@@ -276,7 +260,7 @@ __global__ void __launch_bounds__(256) alt_complex_kernel(AltParams p) {
                 }
             }
         }
-    }
+    });
 }
 
 // ------------------------------------------------------------------ host ----
@@ -284,18 +268,22 @@ constexpr int64_t kMaxAltTableSmem = 96 * 1024;
 
 template <int S, int MODE, bool CPLX>
 static int launch_alt_k(const AltParams& p, cudaStream_t st) {
-    auto kern = CPLX ? alt_complex_kernel<S, MODE> : alt_real_kernel<S, MODE>;
+    const bool wide = column_wide(p.n1, p.n2);
+    void (*kern)(AltParams, ColumnGeom);
+    if constexpr (CPLX)
+        kern = wide ? alt_complex_kernel<S, MODE, int64_t> : alt_complex_kernel<S, MODE, int>;
+    else
+        kern = wide ? alt_real_kernel<S, MODE, int64_t> : alt_real_kernel<S, MODE, int>;
     const int64_t smem = p.v.table_in_smem ? (int64_t)p.v.npts * (S == TIPT_F32C ? 4 : 8) : 0;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return fail_cuda(e, "integrator smem attribute");
     }
-    const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
-    int64_t blocks = (N + 255) / 256;
-    const int64_t cap = (int64_t)num_sms() * 8;
-    if (blocks > cap) blocks = cap;
-    kern<<<(unsigned)blocks, 256, (size_t)smem, st>>>(p);
+    unsigned blocks;
+    const ColumnGeom g = column_geom(p.n0, p.n1, p.n2, 0, p.n0,
+                                     alt_blocks<S, CPLX>() * (int64_t)num_sms(), blocks);
+    kern<<<blocks, 256, (size_t)smem, st>>>(p, g);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "integrator launch");
 }
