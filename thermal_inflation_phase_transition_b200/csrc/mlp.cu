@@ -331,6 +331,7 @@ __global__ void mlp_reduce_kernel(const float* part, int tiles, float* grad) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
     double s = 0.0;
+#pragma unroll 16
     for (int b = 0; b < tiles; ++b) s += (double)part[(int64_t)b * kParams + p];
     grad[p] = (float)s;
 }
@@ -358,7 +359,7 @@ __global__ void mlp_adam_kernel(float* p, const float* g, float* m, float* v,
 }
 
 // ---------------------------------------------------------------- tcgen05 path
-// The same network on the 5th-generation tensor cores.  Operands sit in shared
+// The same network on the 5th-generation tensor cores, the default.  Operands sit in shared
 // memory in the canonical K-major, non-swizzled UMMA layout: a tile of R rows
 // (the M or N extent) is stored as K/8 column chunks, each holding the R rows'
 // 8 consecutive K values (16 bytes) back to back, so an 8 x 8 core matrix is 128
@@ -367,10 +368,6 @@ __global__ void mlp_adam_kernel(float* p, const float* g, float* m, float* v,
 // tile row, column = output feature; one thread issues the MMAs and commits
 // them to an mbarrier that every thread waits on with a time limit.  Warps w
 // and w + 4 read the same 32 TMEM lanes (w % 4) and split the columns.
-//
-// Backward: dW = H^T dZ (M = in, N = out; for the 16-wide input layer
-// dW^T = dZ^T H, M = out, N = 16) into TMEM columns [0, 128); dH = dZ W^T
-// (M = rows, N = in) into columns [128, 256).
 
 __device__ int g_mlp_status = 0;  // TIPT_ERR_TIMEOUT after a bounded wait expired
 constexpr uint64_t kWaitNs = 2000000000ull;
@@ -469,21 +466,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&f)[16]) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(v[j]);
 }
-// ... and 8
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&f)[8]) {
-    uint32_t v[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
-                   "=r"(v[6]), "=r"(v[7])
-                 : "r"(addr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]),
-                   "+r"(v[6]), "+r"(v[7])
-                 :
-                 : "memory");
-#pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[j]);
-}
 // 8 consecutive K values of one row -> one 16-byte store in the canonical layout
 __device__ __forceinline__ void st_chunk(bf16* T, int r, int k0, int R, const float* f) {
     __nv_bfloat162 h[4];
@@ -491,35 +473,13 @@ __device__ __forceinline__ void st_chunk(bf16* T, int r, int k0, int R, const fl
     for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
     *reinterpret_cast<uint4*>(T + cidx(r, k0, R)) = *reinterpret_cast<uint4*>(h);
 }
-// sum over the warp's 32 rows of each of NC columns in butterfly order (rows 16 apart first),
-// halving the columns a lane carries while it can: NC - 1 + log2(32 / NC) shuffles, and the
-// bits of a full butterfly of every column, since each sum pairs the same two values -> s[col]
-template <int NC>
-__device__ __forceinline__ void col_sums(float (&f)[NC], float* s) {
-    const int lane = threadIdx.x & 31;
-    int m = 16;
-#pragma unroll
-    for (int n = NC / 2; n > 0; n /= 2, m /= 2) {
-        const bool up = (lane & m) != 0;
-#pragma unroll
-        for (int j = 0; j < NC / 2; ++j) {
-            if (j >= n) break;
-            const float send = up ? f[j] : f[j + n];
-            f[j] = (up ? f[j + n] : f[j]) + __shfl_xor_sync(0xffffffffu, send, m);
-        }
-    }
-    constexpr int per = 32 / NC;  // lanes that end with the same column
-#pragma unroll
-    for (int b = per / 2; b > 0; b /= 2) f[0] += __shfl_xor_sync(0xffffffffu, f[0], b);
-    if ((lane & (per - 1)) == 0) s[lane / per] = f[0];
-}
-
 // W_l [K][N] (FP32) -> the forward operand B[N][K]: a thread takes 8 inputs of one output, so
 // its loads are independent and coalesced and its store is one 16-byte chunk
 template <int NT>
 __device__ __forceinline__ void stage_w(const float* params, int l, bf16* B) {
     const int K = dim(l), ln = l == 3 ? 5 : 7, N = 1 << ln;
     const float* W = params + w_off(l);
+#pragma unroll 4
     for (int e = threadIdx.x; e < (K / 8) * N; e += NT) {
         const int o = e & (N - 1), i0 = (e >> ln) * 8;
         float f[8];
@@ -528,27 +488,15 @@ __device__ __forceinline__ void stage_w(const float* params, int l, bf16* B) {
         st_chunk(B, o, i0, N, f);
     }
 }
-// ... and the backward operand B[128 inputs][N]
+// src [R][C] -> dst [C][R], both canonical: every 8 x 8 core matrix is 128 consecutive bytes
+// on either side, four of them per transposing load and store of a warp
 template <int NT>
-__device__ __forceinline__ void stage_wt(const float* params, int l, bf16* B) {
-    const int N = dim(l + 1);
-    const float* W = params + w_off(l);
-    for (int e = threadIdx.x; e < 128 * (N / 8); e += NT) {
-        const int i = e & 127, o0 = (e >> 7) * 8;
-        float f[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) f[t] = __ldg(W + i * N + o0 + t);
-        st_chunk(B, i, o0, 128, f);
-    }
-}
-// src [128][C] -> dst [C][128], both canonical: every 8 x 8 core matrix is 128 consecutive
-// bytes on either side, four of them per transposing load and store of a warp
-template <int NT>
-__device__ __forceinline__ void transpose(const bf16* src, bf16* dst, int C) {
+__device__ __forceinline__ void transpose(const bf16* src, bf16* dst, int R, int C) {
     const int lane = threadIdx.x & 31, m = lane >> 3, t = lane & 7;
-    for (int c4 = (threadIdx.x >> 5) * 4; c4 < 2 * C; c4 += NT / 8) {
-        const int core = c4 + m, rg = core & 15, cg = core >> 4;
-        const uint32_t from = smem_u32(src + (cg * 128 + rg * 8 + t) * 8);
+    const int lr = 31 - __clz(R / 8);
+    for (int c4 = (threadIdx.x >> 5) * 4; c4 < (C / 8) << lr; c4 += NT / 8) {
+        const int core = c4 + m, cg = core >> lr, rg = core - (cg << lr);
+        const uint32_t from = smem_u32(src + (cg * R + rg * 8 + t) * 8);
         const uint32_t to = smem_u32(dst + (rg * C + cg * 8 + t) * 8);
         uint32_t v0, v1, v2, v3;
         asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -561,74 +509,78 @@ __device__ __forceinline__ void transpose(const bf16* src, bf16* dst, int C) {
     }
 }
 
-// Threads of a tile: the lane quarter q = warp % 4 fixes a thread's row, the NH = NT / 128
-// warps of a quarter split the columns.  The gradient runs one CTA a tile and few tiles (32
-// for a batch of 4096), so a tile's serial chain is its time: 16 warps.  The forward pass
-// runs up to 2 CTAs an SM of 8 warps.
-constexpr int tc_threads(bool grad) { return grad ? 512 : 256; }
-constexpr int kXin = 128 * 16;  // elements of the input tile
-constexpr int kD3 = 128 * 32;   // elements of the output layer's dZ
 constexpr int kBias = 3 * 128 + 32;
-constexpr int kLossPitch = kOut;
-
-// What bounds it: the latency of a tile's chain of 4 + 4 products -- weights from L2, the
-// products, the epilogues' exponentials and the barriers between.  Weights are staged as
-// 16-byte chunks of independent loads, the next layer's during this layer's product; the
-// activations of all layers stay in shared memory as BF16 and are transposed there for dW
-// (204 KB); pre-activations go to global scratch as [column][row], 128 bytes a warp.
-// Gradient of 4096 rows 155 -> 62 us, 20,000 rows 310 -> 130 us, against 8 warps that staged
-// single elements and recomputed H^T from the pre-activations.
-template <bool GRAD>
-__global__ void __launch_bounds__(tc_threads(GRAD), 1) mlp_tc_kernel(Args a) {
-    constexpr int NT = tc_threads(GRAD), NH = NT / 128;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned char* sm = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    bf16* X = reinterpret_cast<bf16*>(sm);     // input tile [128][16]
-    bf16* H = X + kXin;                        // hidden layers [128][128]: three, or one reused
-    bf16* W0 = H + (GRAD ? 3 : 1) * kTile;     // weights of even layers, backward weights
-    bf16* W1 = W0 + kTile;                     // weights of odd layers, then H^T
-    bf16* DT = W1 + kTile;                     // dZ^T (gradient kernel only, as all below)
-    bf16* D3 = DT + kTile;
-    float* s_bias = reinterpret_cast<float*>(GRAD ? D3 + kD3 : DT);
-    float* s_db = s_bias + kBias;              // [4 lane quarters][128]
-    float* s_loss = s_db + 4 * 128;            // [128 rows][kLossPitch]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(GRAD ? s_loss + 128 * kLossPitch : s_db);
-    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 1);
-    constexpr uint32_t kCols = GRAD ? 256 : 128;
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int q = warp & 3, hf = warp >> 2;
-    const int r = 32 * q + lane;  // tile row = TMEM lane read by this thread
-    const int64_t row0 = (int64_t)blockIdx.x * kRows;
-    const int64_t row = row0 + r;
-    // pre-activation of hidden layer l, column c, row r at zs[l * zl + c * 128]
-    float* zs = a.zsave + row0 * 128 + r;
-    const int64_t zl = a.rows_pad * 128;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(s_tmem)),
-                     "r"(kCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 32) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    // input tile, zero-padded to 16 features: thread = (row, 8-feature chunk)
-    if (tid < 256) {
-        const int rr = tid >> 1, c0 = (tid & 1) * 8;
+template <int NT>
+__device__ __forceinline__ void load_bias(const float* params, float* s_bias) {
+    for (int e = threadIdx.x; e < kBias; e += NT)
+        s_bias[e] = __ldg(params + b_off(e >> 7) + (e & 127));
+}
+// rows [row0, row0 + R) of x, zero-padded to 16 features and to R rows
+template <int R>
+__device__ __forceinline__ void load_x(const Args& a, int64_t row0, bf16* X) {
+    if (threadIdx.x < 2 * R) {
+        const int rr = threadIdx.x >> 1, c0 = (threadIdx.x & 1) * 8;
         float f[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             f[j] = (c0 + j < kIn && row0 + rr < a.rows) ? __ldg(a.x + (row0 + rr) * kIn + c0 + j)
                                                          : 0.0f;
-        st_chunk(X, rr, c0, 128, f);
+        st_chunk(X, rr, c0, R, f);
     }
-    for (int e = tid; e < kBias; e += NT) s_bias[e] = __ldg(a.params + b_off(e >> 7) + (e & 127));
-    stage_w<NT>(a.params, 0, W0);
+}
+// TMEM columns (warp 0) and the barrier (thread 32); the caller's block barrier publishes both
+__device__ __forceinline__ void tc_begin(uint32_t* s_tmem, uint64_t* bar, uint32_t cols) {
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(s_tmem)),
+                     "r"(cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 32) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+}
+__device__ __forceinline__ void tc_end(bool ok, uint32_t tmem, uint32_t cols) {
+    if (!ok && threadIdx.x == 0) atomicExch(&g_mlp_status, (int)TIPT_ERR_TIMEOUT);
+    tc_before();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        tc_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols)
+                     : "memory");
+    }
+}
+
+// ------------------------------------------------------------ forward pass ----
+// Tiles of 128 rows, D lanes = rows, up to 2 CTAs an SM.  The next layer's weights are staged
+// during this layer's product.
+constexpr int kTcFwdThreads = 256;
+constexpr size_t kTcFwdSmem =
+    (kRows * 16 + 3 * kTile) * sizeof(bf16) + kBias * sizeof(float) + 16 + 1024;
+
+__global__ void __launch_bounds__(kTcFwdThreads, 2) mlp_tc_forward_kernel(Args a) {
+    constexpr int NT = kTcFwdThreads;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned char* sm = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    bf16* X = reinterpret_cast<bf16*>(sm);  // input tile [128][16]
+    bf16* H = X + kRows * 16;               // a layer's input and, its product ended, its output
+    bf16* W = H + kTile;                    // weights of even layers, then of odd ones
+    float* s_bias = reinterpret_cast<float*>(W + 2 * kTile);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(s_bias + kBias);
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, q = warp & 3, hf = warp >> 2;
+    const int r = 32 * q + (tid & 31);  // tile row = TMEM lane read by this thread
+    const int64_t row0 = (int64_t)blockIdx.x * kRows;
+    const int64_t row = row0 + r;
+
+    tc_begin(s_tmem, bar, 128);
+    load_x<kRows>(a, row0, X);
+    load_bias<NT>(a.params, s_bias);
+    stage_w<NT>(a.params, 0, W);
     tc_before();
     fence_async_smem();
     __syncthreads();
@@ -637,171 +589,235 @@ __global__ void __launch_bounds__(tc_threads(GRAD), 1) mlp_tc_kernel(Args a) {
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);  // this warp's lane quarter
     uint32_t phase = 0;
     bool ok = true;
-
 #pragma unroll 1
     for (int l = 0; l < 4; ++l) {
-        bf16* hout = H + (GRAD ? l : 0) * kTile;
         if (tid == 0) {
             tc_after();
-            gemm(tmem, l == 0 ? X : (GRAD ? hout - kTile : H), 128, l & 1 ? W1 : W0, dim(l + 1),
-                 dim(l));
+            gemm(tmem, l == 0 ? X : H, 128, W + (l & 1) * kTile, dim(l + 1), dim(l));
             umma_commit(bar);
         }
         // the buffer of layer l - 1's weights is free: its product has ended
-        if (l < 3) stage_w<NT>(a.params, l + 1, l & 1 ? W0 : W1);
-        else if (GRAD) stage_wt<NT>(a.params, 3, W0);
+        if (l < 3) stage_w<NT>(a.params, l + 1, W + (~l & 1) * kTile);
+        ok = mbar_wait(bar, phase);
+        phase ^= 1u;
+        if (!__syncthreads_and(ok)) break;
+        tc_after();
+        if (l < 3) {
+#pragma unroll 1
+            for (int c0 = 64 * hf; c0 < 64 * hf + 64; c0 += 16) {
+                float z[16];
+                tmem_ld16(tl + c0, z);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) z[j] = silu(z[j] + s_bias[128 * l + c0 + j]);
+                st_chunk(H, r, c0, 128, z);
+                st_chunk(H, r, c0 + 8, 128, z + 8);
+            }
+        } else {
+            float y[16];
+            tmem_ld16(tl + 16 * hf, y);
+            if (row < a.rows)
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (16 * hf + j < kOut)
+                        a.y[row * kOut + 16 * hf + j] = y[j] + s_bias[3 * 128 + 16 * hf + j];
+        }
+        tc_before();
+        fence_async_smem();
+        __syncthreads();
+    }
+    tc_end(ok, tmem, 128);
+}
+
+// ---------------------------------------------------------------- gradient ----
+// Tiles of 64 rows with the features on the TMEM lanes: Z^T = W^T H^T (M = 128 outputs, N = 64
+// rows), dH^T = W dZ^T, dW^T = dZ^T H (dW = H^T dZ for the 32-wide output layer), so a bias
+// gradient is a thread's own sum and the stores of dW are coalesced.  An epilogue stores its
+// 16 rows of one feature as chunks of the [features][rows] operand; the [rows][features] one
+// is its transpose in shared memory.  Everything of a tile stays on the SM: weights (read once,
+// the backward ones are transposes), activations and, in TMEM columns [0, 192), the
+// pre-activations; columns [192, 256) hold the output layer and dH^T, [256, 384) dW.
+//
+// What bounds it: the latency of a tile's chain of 4 + 4 products, the exponentials of the
+// epilogues and the barriers between, so few rows a CTA and 16 warps.  (Slices of 64 rows are
+// what the workspace holds.)  Kernel at 4096 rows 155 us -> 31 us, a training step 169 -> 48 us
+// (20,000 rows 322 -> 117 us) against tiles of 128 rows on 8 warps that staged single elements
+// and recomputed H^T from stored pre-activations.
+constexpr int kGT = 512;          // threads
+constexpr int kGR = 64;           // rows of a tile
+constexpr int kGTile = 128 * kGR;  // elements of a [features][rows] operand
+constexpr int kLossPitch = kOut;
+// X, X^T, H^T of three layers, [rows][features], dZ^T, W_0..W_2, W_3 (32 rows of 128, and what
+// the 128-row product reads past them), backward weights
+constexpr int kGOperands = 2 * kGR * 16 + 3 * kGTile + 2 * kGTile + 128 * 16 + 2 * kTile + 5120 + kTile;
+constexpr size_t kTcGradSmem = kGOperands * sizeof(bf16) +
+                               (kBias + 4 * 128 + kGR * kLossPitch) * sizeof(float) + 16 + 1024;
+static_assert(kTcGradSmem <= 227 * 1024, "gradient tile");
+
+__global__ void __launch_bounds__(kGT, 1) mlp_tc_grad_kernel(Args a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned char* sm = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    bf16* X = reinterpret_cast<bf16*>(sm);  // [rows][16]
+    bf16* XT = X + kGR * 16;                // [16][rows]
+    bf16* HT = XT + kGR * 16;               // H_1..H_3 as [128][rows]
+    bf16* HR = HT + 3 * kGTile;             // a layer's input, or dZ, as [rows][features]
+    bf16* DT = HR + kGTile;                 // dZ^T
+    bf16* W0 = DT + kGTile;                 // [128][16]
+    bf16* W1 = W0 + 128 * 16;               // W_1, W_2 as [out][in]
+    bf16* W3 = W1 + 2 * kTile;
+    bf16* WB = W3 + 5120;                   // W_l as [in][out]
+    float* s_bias = reinterpret_cast<float*>(WB + kTile);
+    float* s_db = s_bias + kBias;           // [4 row quarters][128]
+    float* s_loss = s_db + 4 * 128;         // [rows][kLossPitch]
+    uint64_t* bar = reinterpret_cast<uint64_t*>(s_loss + kGR * kLossPitch);
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar + 1);
+    constexpr uint32_t kAcc = 3 * kGR, kDw = 4 * kGR;  // TMEM columns
+
+    const int tid = threadIdx.x, lane = tid & 31, q = (tid >> 5) & 3, hf = tid >> 7;
+    const int r = 32 * q + lane;  // feature = TMEM lane read by this thread
+    const int c0 = 16 * hf;       // its 16 rows of the tile
+    const int64_t row0 = (int64_t)blockIdx.x * kGR;
+
+    tc_begin(s_tmem, bar, 512);
+    load_x<kGR>(a, row0, X);
+    load_bias<kGT>(a.params, s_bias);
+    stage_w<kGT>(a.params, 0, W0);
+    tc_before();
+    fence_async_smem();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = *s_tmem;
+    const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);  // this warp's lane quarter
+    uint32_t phase = 0;
+    bool ok = true;
+    float* part = a.partials + (int64_t)blockIdx.x * kParams;
+    // sums of the tile's rows by the lane quarter of rows, then over the quarters
+    const auto put_dz = [&](float (&g)[16], int N) {
+        st_chunk(DT, r, c0, N, g);
+        st_chunk(DT, r, c0 + 8, N, g + 8);
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s += g[j];
+        s_db[hf * 128 + r] = s;
+    };
+
+#pragma unroll 1
+    for (int l = 0; l < 4; ++l) {
+        if (tid == 0) {
+            tc_after();
+            const bf16* W = l == 0 ? W0 : (l == 3 ? W3 : W1 + (l - 1) * kTile);
+            gemm(tmem + l * kGR, W, l == 3 ? 32 : 128, l == 0 ? X : HR, kGR, dim(l));
+            umma_commit(bar);
+        }
+        if (l < 3) stage_w<kGT>(a.params, l + 1, l == 2 ? W3 : W1 + l * kTile);
+        else transpose<kGT>(W3, WB, 32, 128);
         ok = mbar_wait(bar, phase);
         phase ^= 1u;
         if (!__syncthreads_and(ok)) goto done;
         tc_after();
         if (l < 3) {
-#pragma unroll 1
-            for (int c0 = 16 * hf; c0 < 128; c0 += 16 * NH) {
-                float z[16];
-                tmem_ld16(tl + c0, z);
+            float z[16];
+            tmem_ld16(tl + l * kGR + c0, z);
+            const float b = s_bias[128 * l + r];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) z[j] += s_bias[128 * l + c0 + j];
-                if (GRAD) {
+            for (int j = 0; j < 16; ++j) z[j] = silu(z[j] + b);
+            bf16* H = HT + l * kGTile;
+            st_chunk(H, r, c0, 128, z);
+            st_chunk(H, r, c0 + 8, 128, z + 8);
+            __syncthreads();
+            transpose<kGT>(H, HR, 128, kGR);
+        } else if (q == 0) {
+            // output r of 16 rows; loss terms to s_loss, summed in output order below
+            float y[16];
+            tmem_ld16(tl + kAcc + c0, y);
+            const float b = s_bias[3 * 128 + r];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) zs[l * zl + (c0 + j) * 128] = z[j];
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) z[j] = silu(z[j]);
-                st_chunk(hout, r, c0, 128, z);
-                st_chunk(hout, r, c0 + 8, 128, z + 8);
-            }
-        } else {
-            // output layer: this thread holds row r's outputs [c0, c0 + NY)
-            constexpr int NY = 32 / NH;
-            const int c0 = NY * hf;
-            const bool valid = row < a.rows;
-            float y[NY];
-            if constexpr (NY == 8) tmem_ld8(tl + c0, y);
-            else tmem_ld16(tl + c0, y);
-#pragma unroll
-            for (int j = 0; j < NY; ++j) y[j] += s_bias[3 * 128 + c0 + j];
-            if (a.y && valid)
-#pragma unroll
-                for (int j = 0; j < NY; ++j)
-                    if (c0 + j < kOut) a.y[row * kOut + c0 + j] = y[j];
-            if constexpr (GRAD) {
-                const float* tg = a.tgt + (valid ? row : 0) * kTgt;
-#pragma unroll
-                for (int j = 0; j < NY; ++j) {
-                    const int c = c0 + j;
-                    float d = 0.0f;
-                    if (valid && c < kOut) {
-                        const float yv = y[j];
-                        if (c == 0) {
-                            const float ev = __ldg(tg), ex = __ldg(tg + 1), wg = __ldg(tg + 2);
-                            const float E = expf(fminf(fmaxf(yv, -kClamp), kClamp));
-                            s_loss[r * kLossPitch] = wg * (E * ex - ev * yv);
-                            d = wg * ((fabsf(yv) < kClamp ? E : 0.0f) * ex - ev) * a.inv_norm;
-                        } else {
-                            const float wc = __ldg(tg + 3) * (1.0f / kCurve), f = __ldg(tg + 3 + c);
-                            const float sp = fmaxf(yv, 0.0f) + log1pf(expf(-fabsf(yv)));
-                            s_loss[r * kLossPitch + c] = sp - f * yv;
-                            d = wc * (sigm(yv) - f) * a.inv_norm;
-                        }
+            for (int j = 0; j < 16; ++j) {
+                const int64_t row = row0 + c0 + j;
+                float d = 0.0f;
+                if (r < kOut && row < a.rows) {
+                    const float* tg = a.tgt + row * kTgt;
+                    const float yv = y[j] + b;
+                    float* term = s_loss + (c0 + j) * kLossPitch + r;
+                    if (r == 0) {
+                        const float ev = __ldg(tg), ex = __ldg(tg + 1), wg = __ldg(tg + 2);
+                        const float E = expf(fminf(fmaxf(yv, -kClamp), kClamp));
+                        *term = wg * (E * ex - ev * yv);
+                        d = wg * ((fabsf(yv) < kClamp ? E : 0.0f) * ex - ev) * a.inv_norm;
+                    } else {
+                        const float wc = __ldg(tg + 3) * (1.0f / kCurve), f = __ldg(tg + 3 + r);
+                        const float sp = fmaxf(yv, 0.0f) + log1pf(expf(-fabsf(yv)));
+                        *term = sp - f * yv;
+                        d = wc * (sigm(yv) - f) * a.inv_norm;
                     }
-                    y[j] = d;
                 }
-                st_chunk(D3, r, c0, 128, y);
-                col_sums(y, s_db + q * 128 + c0);
+                y[j] = d;
+            }
+            put_dz(y, 32);
+        }
+        tc_before();
+        fence_async_smem();
+        __syncthreads();
+    }
+    if (tid < kGR && a.loss_rows && row0 + tid < a.rows) {
+        const float wc = __ldg(a.tgt + (row0 + tid) * kTgt + 3) * (1.0f / kCurve);
+        float loss = s_loss[tid * kLossPitch];
+        for (int j = 1; j < kOut; ++j) loss += wc * s_loss[tid * kLossPitch + j];
+        a.loss_rows[row0 + tid] = loss;
+    }
+    transpose<kGT>(X, XT, kGR, 16);
+#pragma unroll 1
+    for (int l = 3; l >= 0; --l) {
+        const int N = dim(l + 1);
+        bf16* Hl = l > 0 ? HT + (l - 1) * kGTile : XT;  // this layer's input
+        if (tid < N)
+            part[b_off(l) + tid] = ((s_db[tid] + s_db[128 + tid]) + s_db[256 + tid]) + s_db[384 + tid];
+        if (l > 0) transpose<kGT>(DT, HR, N, kGR);
+        if (l == 1 || l == 2) transpose<kGT>(W1 + (l - 1) * kTile, WB, 128, 128);
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc_after();
+            if (l > 0) gemm(tmem + kAcc, WB, 128, HR, kGR, N);           // dH^T[in][rows]
+            if (l == 3) gemm(tmem + kDw, Hl, 128, DT, N, kGR);           // dW[in][out]
+            else gemm(tmem + kDw, DT, 128, Hl, l == 0 ? 16 : 128, kGR);  // dW^T[out][in]
+            umma_commit(bar);
+        }
+        ok = mbar_wait(bar, phase);
+        phase ^= 1u;
+        if (!__syncthreads_and(ok)) goto done;
+        tc_after();
+        if (l > 0) {
+            // dZ^T_{l-1} = dH^T * SiLU'(z_{l-1})
+            float g[16], z[16];
+            tmem_ld16(tl + kAcc + c0, g);
+            tmem_ld16(tl + (l - 1) * kGR + c0, z);
+            const float b = s_bias[128 * (l - 1) + r];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) g[j] *= dsilu(z[j] + b);
+            put_dz(g, 128);
+        }
+        for (int k0 = c0; k0 < (l == 3 ? 32 : dim(l)); k0 += 64) {
+            float g[16];
+            tmem_ld16(tl + kDw + k0, g);
+            float* P = part + w_off(l);
+            if (l == 3) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    reinterpret_cast<float4*>(P + r * 32 + k0)[j] =
+                        make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) P[(k0 + j) * 128 + r] = g[j];
             }
         }
         tc_before();
         fence_async_smem();
         __syncthreads();
     }
-    if constexpr (GRAD) {
-        if (hf == 3 && a.loss_rows && row < a.rows) {
-            const float wc = __ldg(a.tgt + row * kTgt + 3) * (1.0f / kCurve);
-            float loss = s_loss[r * kLossPitch];
-            for (int j = 1; j < kOut; ++j) loss += wc * s_loss[r * kLossPitch + j];
-            a.loss_rows[row] = loss;
-        }
-        float* part = a.partials + (int64_t)blockIdx.x * kParams;
-        bf16* D = D3;
-#pragma unroll 1
-        for (int l = 3; l >= 0; --l) {
-            const int N = dim(l + 1);
-            bf16* Hl = l > 0 ? H + (l - 1) * kTile : X;  // this layer's input
-            if (tid < N) part[b_off(l) + tid] = ((s_db[tid] + s_db[128 + tid]) + s_db[256 + tid]) +
-                                                s_db[384 + tid];
-            transpose<NT>(D, DT, N);
-            transpose<NT>(Hl, W1, dim(l));
-            if (l == 1 || l == 2) stage_wt<NT>(a.params, l, W0);
-            fence_async_smem();
-            __syncthreads();
-            if (tid == 0) {
-                tc_after();
-                if (l > 0) {
-                    gemm(tmem, W1, 128, DT, N, 128);       // dW[in][out]
-                    gemm(tmem + 128, D, 128, W0, 128, N);  // dH[rows][in]
-                } else {
-                    gemm(tmem, DT, 128, W1, 16, 128);      // dW^T[out][in]
-                }
-                umma_commit(bar);
-            }
-            ok = mbar_wait(bar, phase);
-            phase ^= 1u;
-            if (!__syncthreads_and(ok)) goto done;
-            tc_after();
-            if (l > 0) {
-                // dZ_{l-1} = dH * SiLU'(z_{l-1}) for row r, over this layer's input
-#pragma unroll 1
-                for (int c0 = 16 * hf; c0 < 128; c0 += 16 * NH) {
-                    float z[16], g[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) z[j] = zs[(l - 1) * zl + (c0 + j) * 128];
-                    tmem_ld16(tl + 128 + c0, g);
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) g[j] *= dsilu(z[j]);
-                    st_chunk(Hl, r, c0, 128, g);
-                    st_chunk(Hl, r, c0 + 8, 128, g + 8);
-                    col_sums(g, s_db + q * 128 + c0);
-                }
-                // dW rows i = r
-#pragma unroll 1
-                for (int c0 = 16 * hf; c0 < N; c0 += 16 * NH) {
-                    float g[16];
-                    tmem_ld16(tl + c0, g);
-                    float4* P = reinterpret_cast<float4*>(part + w_off(l) + r * N + c0);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        P[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
-                }
-                D = Hl;
-            } else if (hf == 0) {
-                // dW^T rows o = r, 16 input columns
-                float g[16];
-                tmem_ld16(tl, g);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) part[w_off(0) + j * 128 + r] = g[j];
-            }
-            tc_before();
-            fence_async_smem();
-            __syncthreads();
-        }
-    }
 done:
-    if (!ok && tid == 0) atomicExch(&g_mlp_status, (int)TIPT_ERR_TIMEOUT);
-    tc_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols)
-                     : "memory");
-    }
+    tc_end(ok, tmem, 512);
 }
-
-// operands, biases and, for the gradient, bias sums and loss terms; 16 bytes of barrier and
-// TMEM address, 1024 of alignment
-constexpr size_t kTcFwdSmem = (kXin + 3 * kTile) * sizeof(bf16) + kBias * sizeof(float) + 16 + 1024;
-constexpr size_t kTcGradSmem = (kXin + 6 * kTile + kD3) * sizeof(bf16) +
-                               (kBias + 4 * 128 + 128 * kLossPitch) * sizeof(float) + 16 + 1024;
-static_assert(kTcGradSmem <= 227 * 1024, "gradient tile");
 
 int g_policy = 0;  // 0 automatic (tcgen05), 1 mma.sync, 2 tcgen05
 
@@ -865,11 +881,11 @@ extern "C" int tipt_mlp_forward(const float* params, const float* x, int64_t row
         if (e != cudaSuccess) return fail_cuda(e, "mlp forward attributes");
         mlp_kernel<false><<<(unsigned)tiles_of(rows), kThreads, kFwdSmem, (cudaStream_t)stream>>>(a);
     } else {
-        e = cudaFuncSetAttribute(mlp_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(mlp_tc_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kTcFwdSmem);
         if (e != cudaSuccess) return fail_cuda(e, "mlp forward attributes");
-        mlp_tc_kernel<false>
-            <<<(unsigned)tiles_of(rows), tc_threads(false), kTcFwdSmem, (cudaStream_t)stream>>>(a);
+        mlp_tc_forward_kernel<<<(unsigned)tiles_of(rows), kTcFwdThreads, kTcFwdSmem,
+                                (cudaStream_t)stream>>>(a);
     }
     e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "mlp forward launch");
@@ -888,29 +904,34 @@ extern "C" int tipt_mlp_grad(const float* params, const float* x, const float* t
     if (workspace_bytes < need)
         return fail(TIPT_ERR_ARG, "workspace of %lld bytes is smaller than the %lld needed",
                     (long long)workspace_bytes, (long long)need);
-    const int64_t tiles = tiles_of(rows);
     Args a{};
     a.params = params;
     a.x = x;
     a.tgt = tgt;
     a.rows = rows;
     a.inv_norm = 1.0f / norm;
-    a.zsave = static_cast<float*>(workspace);
-    a.rows_pad = tiles * kRows;
-    a.partials = a.zsave + 3 * a.rows_pad * 128;
     a.loss_rows = loss_rows;
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
+    int64_t tiles;
     if (g_policy == 1) {
+        tiles = tiles_of(rows);
+        a.zsave = static_cast<float*>(workspace);
+        a.rows_pad = tiles * kRows;
+        a.partials = a.zsave + 3 * a.rows_pad * 128;
         e = cudaFuncSetAttribute(mlp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kGradSmem);
         if (e != cudaSuccess) return fail_cuda(e, "mlp gradient attributes");
         mlp_kernel<true><<<(unsigned)tiles, kThreads, kGradSmem, st>>>(a);
     } else {
-        e = cudaFuncSetAttribute(mlp_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        // two slices per 128 rows and no pre-activations: within the same workspace
+        static_assert(2 * kParams <= 3 * kRows * 128 + kParams, "gradient slices");
+        tiles = (rows + kGR - 1) / kGR;
+        a.partials = static_cast<float*>(workspace);
+        e = cudaFuncSetAttribute(mlp_tc_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kTcGradSmem);
         if (e != cudaSuccess) return fail_cuda(e, "mlp gradient attributes");
-        mlp_tc_kernel<true><<<(unsigned)tiles, tc_threads(true), kTcGradSmem, st>>>(a);
+        mlp_tc_grad_kernel<<<(unsigned)tiles, kGT, kTcGradSmem, st>>>(a);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "mlp gradient launch");
