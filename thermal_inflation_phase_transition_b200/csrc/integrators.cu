@@ -52,15 +52,6 @@ __device__ __forceinline__ double force_d(const AltParams& p, double lap, double
     return __dsub_rn(__dmul_rn(p.inv_a2, lap), __dmul_rn(dv, p.inv_mu2));
 }
 
-template <typename TT>
-__device__ __forceinline__ const TT* stage_alt_table(const AltParams& p, TT* s_tab) {
-    if (p.v.table_in_smem) {
-        for (int q = threadIdx.x; q < p.v.npts; q += blockDim.x) s_tab[q] = (TT)__ldg(p.v.table + q);
-        __syncthreads();
-    }
-    return s_tab;
-}
-
 // Any lattice shape on the column walk (column_walk.cuh); a table goes to shared memory once
 // per resident block.  Bound by the latency of the loads and of the force and noise chains.
 // Resident blocks per SM, measured at 3 / 4 / 5 / 6 (us): complex float32 256^3 overdamped
@@ -76,10 +67,6 @@ constexpr int alt_blocks() {
 // ----------------------------------------------------------------- real ----
 template <int S, int MODE, typename I>
 __global__ void __launch_bounds__(256, (alt_blocks<S, false>())) alt_real_kernel(AltParams p, ColumnGeom g) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    using TT = typename std::conditional<S == TIPT_F32C, float, double>::type;
-    const TT* s_tab = stage_alt_table<TT>(p, reinterpret_cast<TT*>(smem_raw));
-    const double* dtab = p.v.table_in_smem ? reinterpret_cast<const double*>(s_tab) : p.v.table;
     const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
     const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
     // the stored planes of a site: phi, or its hi and lo parts
@@ -97,7 +84,7 @@ __global__ void __launch_bounds__(256, (alt_blocks<S, false>())) alt_real_kernel
             if constexpr (S == TIPT_F64) lap = lap_d(nb[0], p.inv_dx2);
             else lap = lap_f(nb[0], p.inv_dx2);
             const double ph = (double)nb[0][0];
-            const double F = force_d(p, lap, vprime_alt_d(p.v, dtab, ph));
+            const double F = force_d(p, lap, vprime_alt_d(p.v, p.v.table, ph));
             const double z = noisy ? gauss_cos(key) : 0.0;
             if constexpr (MODE == kOD) {
                 static_cast<E*>(p.o[0])[s] =
@@ -117,7 +104,8 @@ __global__ void __launch_bounds__(256, (alt_blocks<S, false>())) alt_real_kernel
         } else {
             float dh, dl;
             stencil_sums(nb[0], nb[1], dh, dl);
-            const float vp = vprime_alt_f(p.v, s_tab, __fadd_rn(nb[0][0], nb[1][0]));
+            const float vp = vprime_alt_f(p.v, RowReader<float, false>{p.v.table},
+                                           __fadd_rn(nb[0][0], nb[1][0]));
             const float z = noisy ? gauss_cos_f(key) : 0.0f;
             float* out0 = static_cast<float*>(p.o[0]);
             float* out1 = static_cast<float*>(p.o[1]);
@@ -143,10 +131,6 @@ __global__ void __launch_bounds__(256, (alt_blocks<S, false>())) alt_real_kernel
 // -------------------------------------------------------------- complex ----
 template <int S, int MODE, typename I>
 __global__ void __launch_bounds__(256, (alt_blocks<S, true>())) alt_complex_kernel(AltParams p, ColumnGeom g) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    using TT = typename std::conditional<S == TIPT_F32C, float, double>::type;
-    const TT* s_tab = stage_alt_table<TT>(p, reinterpret_cast<TT*>(smem_raw));
-    const double* dtab = p.v.table_in_smem ? reinterpret_cast<const double*>(s_tab) : p.v.table;
     const bool zn = p.v.zn_active > 0.5 && p.v.zn_n > 0.5;
     const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
     const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
@@ -172,7 +156,7 @@ __global__ void __launch_bounds__(256, (alt_blocks<S, true>())) alt_complex_kern
                 c[a] = (double)nb[a][0];
             }
             double d1, d2;
-            complex_force<false>(p.v, dtab, c[0], c[1], d1, d2);
+            complex_force<false>(p.v, p.v.table, c[0], c[1], d1, d2);
             const double F[2] = {force_d(p, lap[0], d1), force_d(p, lap[1], d2)};
             double z[2] = {0.0, 0.0};
             if (noisy) gauss_pair(key, z[0], z[1]);
@@ -207,7 +191,7 @@ __global__ void __launch_bounds__(256, (alt_blocks<S, true>())) alt_complex_kern
             }
             float d1, d2;
             if (!zn && (p.v.table_in_smem || p.v.vkind == TIPT_VP_POLY)) {
-                complex_force_v<float>(p.v, s_tab, (float)p.v.tmin, (float)p.v.dinv,
+                complex_force_v<float>(p.v, RowReader<float, false>{p.v.table}, (float)p.v.tmin, (float)p.v.dinv,
                                        __fadd_rn(ch[0], cl[0]), __fadd_rn(ch[1], cl[1]), d1, d2);
             } else {
                 double e1, e2;
@@ -274,25 +258,26 @@ static int launch_alt_k(const AltParams& p, cudaStream_t st) {
         kern = wide ? alt_complex_kernel<S, MODE, int64_t> : alt_complex_kernel<S, MODE, int>;
     else
         kern = wide ? alt_real_kernel<S, MODE, int64_t> : alt_real_kernel<S, MODE, int>;
-    const int64_t smem = p.v.table_in_smem ? (int64_t)p.v.npts * (S == TIPT_F32C ? 4 : 8) : 0;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return fail_cuda(e, "integrator smem attribute");
-    }
     unsigned blocks;
     const ColumnGeom g = column_geom(p.n0, p.n1, p.n2, 0, p.n0,
                                      alt_blocks<S, CPLX>() * (int64_t)num_sms(), blocks);
-    kern<<<blocks, 256, (size_t)smem, st>>>(p, g);
+    kern<<<blocks, 256, 0, st>>>(p, g);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "integrator launch");
 }
 
 template <int MODE, bool CPLX>
 static int launch_alt(int storage, const AltParams& p, cudaStream_t st) {
-    // compensated FP32 on the marching ring where the shape allows (bitwise the
-    // generic kernel's results; kernel_policy 1 forces the generic one)
-    if (storage == TIPT_F32C && kernel_policy() != 1 && alt_march_supported(p, CPLX))
+    // compensated FP32 on the marching ring where the shape allows and it pays (bitwise the
+    // generic kernel's results; kernel_policy 1 forces the generic one).  Rows that are not
+    // whole 128-byte lines are copied one by one (march / generic in us, complex overdamped
+    // 80^3 31 / 13, 112^3 68 / 25, 240^3 239 / 191; real BAOAB 80^3 38 / 22, 208^3 204 / 191,
+    // 240^3 260 / 285), and small lattices do not fill the pipeline (real BAOAB 32^3 14.8 /
+    // 10.6, 64^3 13.1 / 16.0).
+    const int64_t sites = (int64_t)p.n0 * p.n1 * p.n2;
+    const bool pays = p.n2 % 32 == 0 ? sites >= 1 << 18 : !CPLX && sites >= 12 << 20;
+    if (storage == TIPT_F32C && (kernel_policy() == 2 || (kernel_policy() == 0 && pays)) &&
+        alt_march_supported(p, CPLX))
         return launch_alt_march(MODE, CPLX, p, st);
     switch (storage) {
         case TIPT_F64: return launch_alt_k<TIPT_F64, MODE, CPLX>(p, st);

@@ -19,8 +19,8 @@ struct AltParams {
     ComplexStageParams v;  // V' source, Z_N and eps terms (the force fields only)
 };
 
-__device__ __forceinline__ float vprime_alt_f(const ComplexStageParams& v, const float* s_tab,
-                                              float x) {
+template <typename Tab>
+__device__ __forceinline__ float vprime_alt_f(const ComplexStageParams& v, Tab s_tab, float x) {
     if (v.vkind == TIPT_VP_POLY)
         return poly_vprime<float>((float)v.c1, (float)v.c2, (float)v.c3, x);
     if (v.table_in_smem) return lerp_table<float>(s_tab, (float)v.tmin, (float)v.dinv, v.npts - 2, x);

@@ -14,10 +14,10 @@ namespace tipt {
 constexpr int64_t kMaxTableSmemC = 96 * 1024;
 
 template <int S>
-static int launch_complex_generic(const ComplexStageParams& p, int64_t smem, cudaStream_t st) {
+static int launch_complex_generic(const ComplexStageParams& p, cudaStream_t st) {
     const bool th = p.vkind == TIPT_VP_THERMAL;
-    if (p.range) return th ? launch_stage_generic<ComplexSite<S, true, true>>(p, smem, st) : launch_stage_generic<ComplexSite<S, false, true>>(p, smem, st);
-    return th ? launch_stage_generic<ComplexSite<S, true, false>>(p, smem, st) : launch_stage_generic<ComplexSite<S, false, false>>(p, smem, st);
+    if (p.range) return th ? launch_stage_generic<ComplexSite<S, true, true>>(p, st) : launch_stage_generic<ComplexSite<S, false, true>>(p, st);
+    return th ? launch_stage_generic<ComplexSite<S, true, false>>(p, st) : launch_stage_generic<ComplexSite<S, false, false>>(p, st);
 }
 
 int launch_complex_stage(int storage, ComplexStageParams p, cudaStream_t st) {
@@ -25,17 +25,22 @@ int launch_complex_stage(int storage, ComplexStageParams p, cudaStream_t st) {
     const bool no_table = p.vkind == TIPT_VP_POLY || p.vkind == TIPT_VP_THERMAL;
     int64_t tb = no_table ? 0 : (int64_t)p.npts * (storage == TIPT_F32C ? 4 : 8);
     p.table_in_smem = (tb > 0 && tb <= kMaxTableSmemC) ? 1 : 0;
-    const int64_t smem = p.table_in_smem ? tb : 0;
-    if (storage == TIPT_F32C && kernel_policy() != 1) {
+    // The marching kernel needs enough planes of tiles, and more of them where rows are not
+    // whole 128-byte lines (march / generic in us: 64^3 13.7 / 13.2, 96^3 27.8 / 27.6, 128^3 49 /
+    // 60, 256^3 290 / 580; 80^3 49 / 20, 112^3 75 / 43, 144^3 121 / 82, 208^3 247 / 233, 240^3
+    // 322 / 347).
+    const int64_t sites = (int64_t)p.n0 * p.n1 * p.n2;
+    const bool pays = sites >= (p.n2 % 32 == 0 ? 1 << 20 : 12 << 20);
+    if (storage == TIPT_F32C && (kernel_policy() == 2 || (kernel_policy() == 0 && pays))) {
         if (complex_march_supported(p)) return launch_complex_march(p, st);
         if (kernel_policy() == 2)
             return fail(TIPT_ERR_UNSUPPORTED, "the complex marching kernel does not take this "
                         "call (Z_N active, noise arrays, table or shape)");
     }
     switch (storage) {
-        case TIPT_F64: return launch_complex_generic<TIPT_F64>(p, smem, st);
-        case TIPT_F32: return launch_complex_generic<TIPT_F32>(p, smem, st);
-        case TIPT_F32C: return launch_complex_generic<TIPT_F32C>(p, smem, st);
+        case TIPT_F64: return launch_complex_generic<TIPT_F64>(p, st);
+        case TIPT_F32: return launch_complex_generic<TIPT_F32>(p, st);
+        case TIPT_F32C: return launch_complex_generic<TIPT_F32C>(p, st);
     }
     return fail(TIPT_ERR_STORAGE, "unknown storage %d", storage);
 }

@@ -141,8 +141,8 @@ __device__ __forceinline__ float2 v_atleast(float2 a, float m) {
 }
 
 // V'(rho) from the polynomial or the FP32 shared-memory table (R:1923-1930 rule).
-template <typename V>
-__device__ __forceinline__ V cvprime_v(const ComplexStageParams& p, const float* s_tab, V x,
+template <typename V, typename Tab>
+__device__ __forceinline__ V cvprime_v(const ComplexStageParams& p, Tab s_tab, V x,
                                        float tmin, float dinv) {
     if (p.vkind == TIPT_VP_POLY) {
         const V d = v_fma(v_mul(v_mul(vs<V>((float)p.c3), x), x), x, v_mul(vs<V>((float)p.c1), x));
@@ -163,8 +163,8 @@ __device__ __forceinline__ V cvprime_v(const ComplexStageParams& p, const float*
 // operations as the dispatching form's branches).
 enum : int { kCsrcAny = 0, kCsrcTab = 1, kCsrcTabEps = 2 };
 
-template <typename V, int SRC = kCsrcAny>
-__device__ __forceinline__ void complex_force_v(const ComplexStageParams& p, const float* s_tab,
+template <typename V, int SRC = kCsrcAny, typename Tab>
+__device__ __forceinline__ void complex_force_v(const ComplexStageParams& p, Tab s_tab,
                                                 float tmin, float dinv, V p1, V p2, V& d1,
                                                 V& d2) {
     const V r2 = v_atleast(v_fma(p1, p1, v_mul(p2, p2)), 1e-36f);

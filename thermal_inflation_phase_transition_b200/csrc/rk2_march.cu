@@ -1559,7 +1559,7 @@ static bool geometry(int storage, const RealStageParams& p, int64_t smem_table, 
                          2 * layout_planes(storage), smem_table, g, smem);
 }
 
-bool march_supported(int storage, const RealStageParams& p) {
+bool march_supported(int storage, const RealStageParams& p, int* warps) {
     if (storage != TIPT_F32C && storage != TIPT_F64 && storage != TIPT_F32) return false;
     const uintptr_t a = reinterpret_cast<uintptr_t>(p.phi) | reinterpret_cast<uintptr_t>(p.pi) |
                         reinterpret_cast<uintptr_t>(p.phi_out) |
@@ -1568,7 +1568,14 @@ bool march_supported(int storage, const RealStageParams& p) {
     MarchGeom g;
     int64_t smem;
     int64_t tb = p.table_in_smem ? (int64_t)p.npts * (storage == TIPT_F32C ? 4 : 8) : 0;
-    return geometry(storage, p, tb, g, smem);
+    if (!geometry(storage, p, tb, g, smem)) return false;
+    if (warps) {
+        const int w = g.TJ * (p.n2 / 4) / 32;
+        const int64_t by_smem = kSmemPerSm / (smem_need(g) + kSmemReserve);
+        const int64_t by_regs = 65536 / (kMarchRegs * 32 * (w + 1));
+        *warps = w * (int)(by_smem < by_regs ? by_smem : by_regs);
+    }
+    return true;
 }
 
 // How the work is split over `ctas` CTAs (MarchRuns), by the planes that the busiest

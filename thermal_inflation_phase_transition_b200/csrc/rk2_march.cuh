@@ -5,7 +5,8 @@
 
 namespace tipt {
 
-bool march_supported(int storage, const RealStageParams& p);
+// warps: consumer warps an SM would run.
+bool march_supported(int storage, const RealStageParams& p, int* warps = nullptr);
 int launch_march(int storage, const RealStageParams& p, int64_t smem_table, cudaStream_t st);
 
 // Batched ensemble: the replicas rids[0..n_rids) of one 3-D shape class on the

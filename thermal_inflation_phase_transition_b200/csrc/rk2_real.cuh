@@ -127,7 +127,7 @@ __device__ __forceinline__ double staged_value(const RealStageParams& p, const d
                                                int q) {
     if (p.vkind == TIPT_VP_TABLE) return __ldg(p.table + q);
     const double va = __ldg(a + q), vb = __ldg(a + p.npts + q);
-    return va + w * (vb - va);
+    return __fma_rn(w, __dsub_rn(vb, va), va);  // as RowReader
 }
 
 template <typename TT>
@@ -161,7 +161,25 @@ __device__ __forceinline__ void stage_table_pairs(const RealStageParams& p, floa
     __syncthreads();
 }
 
-// V'(x) in FP64 from the staged row, the global 1-D table, or the polynomial.
+// The row of a table source read in place (after the schedule is resolved).
+template <typename R, bool TWO>
+__device__ __forceinline__ RowReader<R, TWO> row_reader(const RealStageParams& p) {
+    if constexpr (TWO) {
+        __shared__ RowBlend s_row;
+        if (threadIdx.x == 0) {
+            int it;
+            table2d_row(p, it, s_row.w);
+            s_row.a = p.table + (int64_t)it * p.npts;
+        }
+        __syncthreads();
+        return RowReader<R, true>{&s_row, p.npts};
+    } else {
+        return RowReader<R, false>{p.table};
+    }
+}
+
+// V'(x) in FP64 from the staged row, the global 1-D table, or the polynomial; from a row
+// read in place in the second form.
 // TH = false compiles the thermal branch out (see vprime_v).
 template <bool TH = true>
 __device__ __forceinline__ double vprime_d(const RealStageParams& p, const double* s_tab, double x) {
@@ -169,6 +187,13 @@ __device__ __forceinline__ double vprime_d(const RealStageParams& p, const doubl
     if (TH && p.vkind == TIPT_VP_THERMAL) return thermal_vprime_inline(p.th, x);
     const double* t = p.table_in_smem ? s_tab : p.table;
     return lerp_table<double>(t, p.tmin, p.dinv, p.npts - 2, x);
+}
+template <bool TH = true, bool TWO>
+__device__ __forceinline__ double vprime_d(const RealStageParams& p,
+                                           const RowReader<double, TWO>& row, double x) {
+    if (!TWO && p.vkind == TIPT_VP_POLY) return poly_vprime<double>(p.c1, p.c2, p.c3, x);
+    if (TH && p.vkind == TIPT_VP_THERMAL) return thermal_vprime_inline(p.th, x);
+    return lerp_table<double>(row, p.tmin, p.dinv, p.npts - 2, x);
 }
 
 // V'(x) in FP32 (F32C storage) for a lane vector: the polynomial, the float
@@ -230,9 +255,9 @@ __device__ __forceinline__ F32CConst f32c_const(const RealStageParams& p) {
 
 // TH = false compiles the thermal branch out (kernels launched only for the
 // polynomial and table sources keep their register budget).
-template <typename V, bool TH = true>
-__device__ __forceinline__ V vprime_v(const RealStageParams& p, const F32CConst& kc,
-                                      const float* s_tab, V x) {
+template <typename V, bool TH = true, typename Tab>
+__device__ __forceinline__ V vprime_v(const RealStageParams& p, const F32CConst& kc, Tab s_tab,
+                                      V x) {
     constexpr int NL = sizeof(V) / sizeof(float);
     if (p.vkind == TIPT_VP_POLY) {
         const V d = v_fma(v_mul(v_mul(kvec<V>(p.k2.c3), x), x), x, v_mul(kvec<V>(p.k2.c1), x));
@@ -278,8 +303,8 @@ __device__ __forceinline__ double force_d(const RealStageParams& p, double lap, 
 }
 // phi~ = phi + h1 pi is linear in the state, so its Laplacian is lap + h1 lap(pi): no
 // midpoint value per neighbour.
-template <bool TH = true>
-__device__ __forceinline__ void update_f64(const RealStageParams& p, const double* s_tab,
+template <bool TH = true, typename Tab>
+__device__ __forceinline__ void update_f64(const RealStageParams& p, const Tab& s_tab,
                                            const double ph[7], const double pv[7], double noise,
                                            double& phi_new, double& pi_new) {
     const double c = ph[0];
@@ -324,8 +349,8 @@ __device__ __forceinline__ float midpoint_f32_bits(const P& p, float ph, float p
 }
 
 // The update from the stencils of phi and phi~.
-template <bool TH = true>
-__device__ __forceinline__ void update_f32_mid(const RealStageParams& p, const double* s_tab,
+template <bool TH = true, typename Tab>
+__device__ __forceinline__ void update_f32_mid(const RealStageParams& p, const Tab& s_tab,
                                                const float ph[7], const float pt[7], float pv,
                                                double noise, float& phi_new, float& pi_new) {
     const double c = (double)ph[0], ct = (double)pt[0], v = (double)pv;
@@ -336,15 +361,6 @@ __device__ __forceinline__ void update_f32_mid(const RealStageParams& p, const d
     const double k2 = force_d(p, lap2, pit, vprime_d<TH>(p, s_tab, ct));
     phi_new = __double2float_rn(__fma_rn(p.h2, pit, c));
     pi_new = __double2float_rn(__dadd_rn(v, __fma_rn(p.h2, k2, noise)));
-}
-template <bool TH = true>
-__device__ __forceinline__ void update_f32(const RealStageParams& p, const double* s_tab,
-                                           const float ph[7], const float pv[7], double noise,
-                                           float& phi_new, float& pi_new) {
-    float pt[7];
-#pragma unroll
-    for (int q = 0; q < 7; ++q) pt[q] = midpoint_f32(p, ph[q], pv[q]);
-    update_f32_mid<TH>(p, s_tab, ph, pt, pv[0], noise, phi_new, pi_new);
 }
 
 // -------------------------------------------------------------- F32C ----
@@ -398,9 +414,9 @@ __device__ __forceinline__ F32CPre<V> pre_f32c_vp(const RealStageParams& p, V ph
     return r;
 }
 
-template <typename V, bool TH = true>
+template <typename V, bool TH = true, typename Tab>
 __device__ __forceinline__ F32CPre<V> pre_f32c(const RealStageParams& p, const F32CConst& kc,
-                                               const float* s_tab, V phh, V phl, V pih, V pil) {
+                                               const Tab& s_tab, V phh, V phl, V pih, V pil) {
     return pre_f32c_vp<V>(p, phh, phl, pih, pil,
                           [&](V x) { return vprime_v<V, TH>(p, kc, s_tab, x); });
 }
@@ -443,9 +459,9 @@ __device__ __forceinline__ void post_f32c(const RealStageParams& p, const F32CIn
     ff_add1(x.pih, x.pil, v_fma(h2h, k2, kick), pih, pil);
 }
 
-template <typename V, bool TH = true>
+template <typename V, bool TH = true, typename Tab>
 __device__ __forceinline__ void update_f32c(const RealStageParams& p, const F32CConst& kc,
-                                            const float* s_tab, const F32CIn<V>& x, V kick,
+                                            const Tab& s_tab, const F32CIn<V>& x, V kick,
                                             V& phh, V& phl, V& pih, V& pil) {
     const F32CPre<V> pre = pre_f32c<V, TH>(p, kc, s_tab, x.phh, x.phl, x.pih, x.pil);
     post_f32c<V>(p, x, pre, kick, phh, phl, pih, pil);

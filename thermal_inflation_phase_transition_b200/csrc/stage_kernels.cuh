@@ -30,8 +30,7 @@ __global__ void __launch_bounds__(256, 4) stage_generic(typename M::Params p_in,
     M::prepare(p);
     using E = typename M::E;
     RangeAcc racc;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (p.table_in_smem) M::stage(p, smem_raw);
+    const auto row = M::row(p);
     const F32CConst kc = stage_consts(p);
     const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
     walk_columns<E, M::NV, I>(
@@ -41,22 +40,18 @@ __global__ void __launch_bounds__(256, 4) stage_generic(typename M::Params p_in,
             M::load(p, s, N, raw);
             M::values(p, raw, v);
         },
-        [&](int64_t s, const E (&nb)[M::NV][7]) { M::update(p, kc, smem_raw, nb, s, N, racc); });
+        [&](int64_t s, const E (&nb)[M::NV][7]) { M::update(p, kc, row, nb, s, N, racc); });
     if constexpr (M::RG) racc.flush(p.range);
 }
 
 // ----------------------------------------------------------------- launch ---
 template <class M>
-static int launch_stage_generic(const typename M::Params& p, int64_t smem, cudaStream_t st) {
+static int launch_stage_generic(const typename M::Params& p, cudaStream_t st) {
     auto kern = column_wide(p.n1, p.n2) ? stage_generic<M, int64_t> : stage_generic<M, int>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail_cuda(e, "stage_generic smem attribute");
-    }
     unsigned blocks;
     const ColumnGeom g = column_geom(p.n0, p.n1, p.n2, stage_begin(p), stage_end(p),
                                      4 * (int64_t)num_sms(), blocks);
-    kern<<<blocks, 256, (size_t)smem, st>>>(p, g);
+    kern<<<blocks, 256, 0, st>>>(p, g);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "stage_generic launch");
 }

@@ -29,11 +29,15 @@ __device__ __forceinline__ void complex_noise(const ComplexStageParams& p, uint6
 }
 
 // ------------------------------------------------------------ real field ---
-template <int S_, bool TH, bool RG_>
+// What a real stage is compiled for: a 1-D table or the polynomial, a 2-D table, thermal V'.
+enum : int { kSrcRow = 0, kSrcRow2, kSrcThermal };
+
+template <int S_, int SRC, bool RG_>
 struct RealSite {
+    static constexpr bool TH = SRC == kSrcThermal;
     using Params = RealStageParams;
     using E = typename std::conditional<S_ == TIPT_F64, double, float>::type;
-    using TT = typename std::conditional<S_ == TIPT_F32C, float, double>::type;  // staged row
+    using TT = typename std::conditional<S_ == TIPT_F32C, float, double>::type;  // the row is read in
     static constexpr int S = S_;
     static constexpr bool RG = RG_;
     static constexpr int NR = S == TIPT_F32C ? 4 : 2;  // phi, pi; with F32C each hi, lo
@@ -43,8 +47,9 @@ struct RealSite {
         resolve_schedule(p);
         if constexpr (RG) reset_next_range(p);
     }
-    static __device__ __forceinline__ void stage(const Params& p, void* s_tab) {
-        stage_table<TT>(p, static_cast<TT*>(s_tab));
+    using Row = RowReader<TT, SRC == kSrcRow2>;
+    static __device__ __forceinline__ Row row(const Params& p) {
+        return row_reader<TT, SRC == kSrcRow2>(p);
     }
     template <typename I>
     static __device__ __forceinline__ void load(const Params& p, I s, int64_t N, E raw[NR]) {
@@ -71,7 +76,7 @@ struct RealSite {
         }
     }
     static __device__ __forceinline__ void update(const Params& p, const F32CConst& kc,
-                                                  const void* s_tab, const E nb[NV][7],
+                                                  const Row& tab, const E nb[NV][7],
                                                   int64_t s, int64_t N, RangeAcc& racc) {
         const uint64_t site = (uint64_t)(s + p.site_offset);
         E* po = static_cast<E*>(p.phi_out);
@@ -86,7 +91,7 @@ struct RealSite {
             x.pih = nb[2][0];
             x.pil = nb[3][0];
             float a, b, c, d;
-            update_f32c<float, TH>(p, kc, static_cast<const float*>(s_tab), x,
+            update_f32c<float, TH>(p, kc, tab, x,
                                    site_kick_f32c(p, kc, site), a, b, c, d);
             po[s] = a;
             po[N + s] = b;
@@ -96,7 +101,6 @@ struct RealSite {
         } else {
             E a, b;
             const double noise = site_noise<E>(p, site);
-            const double* tab = static_cast<const double*>(s_tab);
             if constexpr (S == TIPT_F64) {
                 update_f64<TH>(p, tab, nb[0], nb[1], noise, a, b);
                 if constexpr (RG) racc.fold_d(a);
@@ -124,11 +128,8 @@ struct ComplexSite {
     static __device__ __forceinline__ void prepare(Params& p) {
         if constexpr (RG) reset_range_words(p.range_next);
     }
-    static __device__ __forceinline__ void stage(const Params& p, void* s_tab) {
-        for (int q = threadIdx.x; q < p.npts; q += blockDim.x)
-            static_cast<TT*>(s_tab)[q] = (TT)__ldg(p.table + q);
-        __syncthreads();
-    }
+    using Row = RowReader<TT, false>;
+    static __device__ __forceinline__ Row row(const Params& p) { return Row{p.table}; }
     template <typename I>
     static __device__ __forceinline__ void load(const Params& p, I s, int64_t N, E raw[NR]) {
 #pragma unroll
@@ -157,7 +158,7 @@ struct ComplexSite {
         }
     }
     static __device__ __forceinline__ void update(const Params& p, const F32CConst&,
-                                                  const void* s_tab, const E nb[NV][7],
+                                                  const Row& tab, const E nb[NV][7],
                                                   int64_t s, int64_t N, RangeAcc& racc) {
         if constexpr (S == TIPT_F32C) {
             // planar {hi, lo} fields; FP32 forces, float-float state updates
@@ -168,7 +169,6 @@ struct ComplexSite {
                 in.ch[f] = nb[2 * f][0];
                 in.cl[f] = nb[2 * f + 1][0];
             }
-            const float* ftab = static_cast<const float*>(s_tab);
             const float h1 = (float)p.h1;
             // The Z_N force of the reference form (C:2152-2158) grows like 1/rho
             // near the origin and amplifies FP32 rounding, so with Z_N active (or a
@@ -178,7 +178,7 @@ struct ComplexSite {
                                     (p.table_in_smem || p.vkind == TIPT_VP_POLY);
             auto force = [&](float q1, float q2, int which, float& d1, float& d2) {
                 if (fp32_force) {
-                    complex_force_v<float>(p, ftab, (float)p.tmin, (float)p.dinv, q1, q2, d1, d2);
+                    complex_force_v<float>(p, tab, (float)p.tmin, (float)p.dinv, q1, q2, d1, d2);
                 } else {
                     double q1d = (double)nb[0][0] + (double)nb[1][0];
                     double q2d = (double)nb[2][0] + (double)nb[3][0];
@@ -212,7 +212,6 @@ struct ComplexSite {
             // FP64 arithmetic after the neighbour sums.  The Laplacian of phi~ = phi + h1 pi
             // is lap + h1 lap(pi); float32 storage takes it from the float32 phi~ and rounds
             // the midpoint's pi, as the reference stores them (see update_f32).
-            const double* tab = p.table_in_smem ? static_cast<const double*>(s_tab) : p.table;
             const auto lap_of = [&](const E v[7], double c) {
                 const E s6 = v[1] + v[2] + v[3] + v[4] + v[5] + v[6];
                 return __dmul_rn(__fma_rn(-6.0, c, (double)s6), p.inv_dx2);
@@ -233,12 +232,12 @@ struct ComplexSite {
                 }
             }
             double d[2], pt[2], n[2];
-            complex_force<TH>(p, tab, c[0], c[1], d[0], d[1]);
+            complex_force<TH>(p, p.table, c[0], c[1], d[0], d[1]);
 #pragma unroll
             for (int a = 0; a < 2; ++a)
                 pt[a] = (double)(E)(c[2 + a] + p.h1 * (p.inv_a2 * lap[a] - p.eta * c[2 + a] -
                                                        d[a] * p.inv_mu2));
-            complex_force<TH>(p, tab, q[0], q[1], d[0], d[1]);
+            complex_force<TH>(p, p.table, q[0], q[1], d[0], d[1]);
             complex_noise<E>(p, (uint64_t)s, n[0], n[1]);
             E o[2];
 #pragma unroll

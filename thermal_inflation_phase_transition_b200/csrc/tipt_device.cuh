@@ -451,8 +451,30 @@ __device__ __forceinline__ double rn_mul(double a, double b) { return __dmul_rn(
 __device__ __forceinline__ float rn_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double rn_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// A V' row read from the FP64 table in global memory, in the type R it would be staged in: the
+// 1-D table, or (TWO) the blend of a 2-D table's rows a and a + npts.
+template <typename R, bool TWO>
+struct RowReader {
+    const double* a;
+    __device__ __forceinline__ R operator[](int q) const { return (R)__ldg(a + q); }
+};
+struct RowBlend {
+    const double* a;
+    double w;
+};
 template <typename R>
-__device__ __forceinline__ R lerp_table(const R* __restrict__ t, R tmin, R dinv, int last, R x) {
+struct RowReader<R, true> {
+    const RowBlend* s;  // in shared memory: the stages have no register to spare
+    int npts;
+    __device__ __forceinline__ R operator[](int q) const {
+        const double* a = s->a + q;
+        const double va = __ldg(a);
+        return (R)__fma_rn(s->w, __dsub_rn(__ldg(a + npts), va), va);
+    }
+};
+
+template <typename R, typename Tab>
+__device__ __forceinline__ R lerp_table(Tab t, R tmin, R dinv, int last, R x) {
     const R fidx = rn_mul(rn_sub(x, tmin), dinv);
     R c = fidx > R(0) ? fidx : R(0);
     c = c < R(last) ? c : R(last);
@@ -476,8 +498,8 @@ __device__ __forceinline__ void vset(float2& v, int l, float x) {
 __device__ __forceinline__ float v_add_rz(float a, float b) { return __fadd_rz(a, b); }
 __device__ __forceinline__ float2 v_add_rz(float2 a, float2 b) { return __fadd2_rz(a, b); }
 
-template <typename V>
-__device__ __forceinline__ V lerp_table_f32(const float* s_tab, V fidx, float last) {
+template <typename V, typename Tab>
+__device__ __forceinline__ V lerp_table_f32(Tab s_tab, V fidx, float last) {
     constexpr int NL = sizeof(V) / sizeof(float);
     V c;
 #pragma unroll
