@@ -55,15 +55,22 @@ def test_observe_counts(storage, shift):
 
 @pytest.mark.parametrize("storage", ["f64", "f32c"])
 def test_shared_chunks(storage):
-    """use_march off: every replica on the work-list; the graph's branches against one stream."""
+    """use_march off: every replica on the work-list; on: the 3-D classes on the
+    work-list kernel, or under policy 2 on the marching stage; the graph's branches against one stream."""
     specs = [EN.ReplicaSpec(s, 1.0, 0.7, seed=n) for n, s in
              enumerate([(16, 16, 16), (31, 7, 9), (128, 128, 1), (50, 49, 1), (96, 32, 33)])]
     out = []
-    for chunk, march, graphs in ((1 << 20, False, False), (8192, False, True), (250, False, True),
-                                 (8192, True, True)):
-        e = EN.Ensemble(specs, storage=storage, chunk_sites=chunk, use_march=march, check_every=4,
-                        retire_frac=1.0, stop_frac=0.01)
-        first = e.run(8, use_graphs=graphs)
+    for chunk, march, graphs, policy in (
+            (1 << 20, False, False, 0), (8192, False, True, 0), (250, False, True, 0),
+            (8192, True, True, 0), (8192, True, False, 0), (8192, True, True, 2),
+            (8192, True, False, 2)):
+        L.set_kernel_policy(policy)
+        try:
+            e = EN.Ensemble(specs, storage=storage, chunk_sites=chunk, use_march=march,
+                            check_every=4, retire_frac=0.51, stop_frac=0.01)
+            first = e.run(12, use_graphs=graphs)
+        finally:
+            L.set_kernel_policy(0)
         out.append((first, e.frac.cpu().numpy(), e.phi[0].clone(), e.pi[0].clone()))
     for o in out[1:]:
         np.testing.assert_array_equal(out[0][0], o[0])

@@ -37,6 +37,12 @@ struct EnsParams {
     const tipt_replica* reps;
     const tipt_chunk* chunks;
     int n_chunks;
+    // a shape class instead of a chunk list: replicas rids[0..*n_rids), kClassChunk sites a
+    // chunk, cpr chunks a replica
+    const int32_t* rids;
+    const int32_t* n_rids;
+    int cpr;
+    uint32_t m1, m2;                     // tipt_replica's multipliers of the class
     int pieces;                          // blocks that share a chunk
     const int32_t* active;
     double h1, h2, inv_dx2, eta, inv_mu2, inv_a2;
@@ -49,17 +55,32 @@ struct EnsParams {
 // x m / 2^32 = x/d + x e / (d 2^32) with e = m d - 2^32 < d); m = 0 means d = 1.
 __device__ __forceinline__ uint32_t fdiv(uint32_t x, uint32_t m) { return m ? __umulhi(x, m) : x; }
 
-template <int S>
+constexpr int kClassChunk = 8192;
+
+template <int S, bool CLASS>
 __global__ void __launch_bounds__(256) ensemble_stage_kernel(EnsParams e) {
     const uint64_t step = e.step + (e.ctr ? *e.ctr + (unsigned long long)e.offset : 0ull);
     // Blocks that share a chunk take its 256-thread passes in turn.
     const int stride = e.pieces * (int)blockDim.x;
-    for (int64_t item = blockIdx.x; item < (int64_t)e.n_chunks * e.pieces; item += gridDim.x) {
+    const int n_chunks = CLASS && e.n_rids ? *e.n_rids * e.cpr : e.n_chunks;
+    for (int64_t item = blockIdx.x; item < (int64_t)n_chunks * e.pieces; item += gridDim.x) {
         const int c = (int)(item / e.pieces);
         const int t0 = (int)(item - (int64_t)c * e.pieces) * (int)blockDim.x + (int)threadIdx.x;
-        const tipt_chunk ch = e.chunks[c];
+        tipt_chunk ch;
+        if constexpr (CLASS) {
+            ch.replica = e.rids[c / e.cpr];
+            ch.begin = (int64_t)(c % e.cpr) * kClassChunk;
+        } else {
+            ch = e.chunks[c];
+        }
         if (!e.active[ch.replica]) continue;
-        const tipt_replica rp = e.reps[ch.replica];
+        tipt_replica rp = e.reps[ch.replica];
+        if constexpr (CLASS) {
+            const int64_t left = (int64_t)rp.n0 * rp.n1 * rp.n2 - ch.begin;
+            ch.count = left < kClassChunk ? (int32_t)left : kClassChunk;
+            rp.m1 = e.m1;
+            rp.m2 = e.m2;
+        }
         // the replica as a single lattice with a polynomial V' and hash noise
         RealStageParams p;
         memset(&p, 0, sizeof(p));
@@ -287,6 +308,25 @@ __global__ void __cluster_dims__(kObsCta, 1, 1) __launch_bounds__(kObsThreads)
     }
 }
 
+// Few chunks are shared between blocks until eight blocks an SM have work: 128 chunks of
+// 8192 sites (64 replicas of 128^2) 33 us on one block each -> 16 us.
+static int stage_grid(EnsParams& e) {
+    const int resident = num_sms() * 8;
+    const int per = e.n_chunks < resident ? resident / e.n_chunks : 1;
+    e.pieces = per < 16 ? per : 16;
+    return e.n_chunks < resident ? e.n_chunks * e.pieces : resident;
+}
+
+// Whether the marching stage is the faster one for n_rids replicas of a class: a launch takes
+// 60 us however little it has to do, and rows that are not whole 128-byte lines are copied one
+// by one (march / work-list kernel in us a step: 64 x 32^3 61 / 31; 4, 16, 64 x 64^3 72 / 18,
+// 74 / 71, 145 / 250; 4, 16 x 96^3 61 / 54, 116 / 202; 64 x 48^3 420 / 109, 64 x 80^3 676 / 494).
+static bool class_march_pays(int32_t n_rids, int32_t n0, int32_t n1, int32_t n2) {
+    const int64_t n = (int64_t)n0 * n1 * n2;
+    if (n * (n1 > n2 ? n1 : n2) >= (1ll << 32)) return true;  // 32-bit site decomposition
+    return n2 % 32 == 0 && n_rids * n >= 4 << 20;
+}
+
 }  // namespace tipt
 
 using namespace tipt;
@@ -322,14 +362,12 @@ extern "C" int tipt_ensemble_step(int storage, const void* phi, const void* pi, 
     e.step = sp->noise_step;
     e.ctr = reinterpret_cast<const unsigned long long*>(counter);
     e.offset = offset;
-    // few chunks are shared between blocks until eight blocks an SM have work: 128 chunks of
-    // 8192 sites (64 replicas of 128^2) 33 us on one block each -> 16 us
-    const int resident = num_sms() * 8;
-    e.pieces = n_chunks < resident ? (resident / n_chunks < 16 ? resident / n_chunks : 16) : 1;
-    const int grid = n_chunks < resident ? n_chunks * e.pieces : resident;
+    e.rids = nullptr;
+    e.n_rids = nullptr;
+    const int grid = stage_grid(e);
     cudaStream_t st = (cudaStream_t)stream;
-    if (storage == TIPT_F64) ensemble_stage_kernel<TIPT_F64><<<grid, 256, 0, st>>>(e);
-    else ensemble_stage_kernel<TIPT_F32C><<<grid, 256, 0, st>>>(e);
+    if (storage == TIPT_F64) ensemble_stage_kernel<TIPT_F64, false><<<grid, 256, 0, st>>>(e);
+    else ensemble_stage_kernel<TIPT_F32C, false><<<grid, 256, 0, st>>>(e);
     cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? TIPT_OK : fail_cuda(err, "ensemble_stage launch");
 }
@@ -359,9 +397,10 @@ extern "C" int tipt_ensemble_observe(int storage, const void* phi, int64_t n_tot
     return err == cudaSuccess ? TIPT_OK : fail_cuda(err, "ensemble_observe launch");
 }
 
-// The replicas of one 3-D shape class in compensated FP32 on the marching stage
-// (shared-memory tiles, TMA/bulk-copy ring): bitwise the same step as
-// tipt_ensemble_step for those replicas.
+// The replicas of one 3-D shape class in compensated FP32, bitwise the step of
+// tipt_ensemble_step for them, on the marching stage (shared-memory tiles, TMA/bulk-copy
+// ring) where it pays, else on the work-list kernel over the class (kernel policy 2: always
+// the marching stage).
 extern "C" int tipt_ensemble_step_march(const void* phi, const void* pi, void* phi_out,
                                         void* pi_out, int64_t n_total,
                                         const tipt_replica* replicas, const int32_t* rids,
@@ -380,6 +419,42 @@ extern "C" int tipt_ensemble_step_march(const void* phi, const void* pi, void* p
     const uintptr_t a = reinterpret_cast<uintptr_t>(phi) | reinterpret_cast<uintptr_t>(pi) |
                         reinterpret_cast<uintptr_t>(phi_out) | reinterpret_cast<uintptr_t>(pi_out);
     if (a % 16 || (n_total * 4) % 16) return fail(TIPT_ERR_ALIGN, "packed buffers must be 16-byte aligned");
+    if (kernel_policy() != 2 && !class_march_pays(n_rids, n0, n1, n2)) {
+        const int64_t cpr = ((int64_t)n0 * n1 * n2 + kClassChunk - 1) / kClassChunk;
+        if (cpr * n_rids <= 0x7FFFFFFF) {
+            const auto magic = [](uint32_t d) {
+                return d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d);
+            };
+            EnsParams e;
+            memset(&e, 0, sizeof(e));
+            e.phi = phi;
+            e.pi = pi;
+            e.phi_out = phi_out;
+            e.pi_out = pi_out;
+            e.n_total = n_total;
+            e.reps = replicas;
+            e.n_chunks = (int)(cpr * n_rids);
+            e.rids = rids;
+            e.n_rids = n_rids_dev;
+            e.cpr = (int)cpr;
+            e.m1 = magic((uint32_t)n1);
+            e.m2 = magic((uint32_t)n2);
+            e.active = active;
+            e.h1 = 0.5 * sp->dt;
+            e.h2 = sp->dt;
+            e.inv_dx2 = 1.0 / (sp->dx * sp->dx);
+            e.eta = sp->eta_eff;
+            e.inv_mu2 = 1.0 / (sp->mu * sp->mu);
+            e.inv_a2 = sp->inv_a2;
+            e.step = sp->noise_step;
+            e.ctr = reinterpret_cast<const unsigned long long*>(counter);
+            e.offset = offset;
+            const int grid = stage_grid(e);
+            ensemble_stage_kernel<TIPT_F32C, true><<<grid, 256, 0, (cudaStream_t)stream>>>(e);
+            cudaError_t err = cudaGetLastError();
+            return err == cudaSuccess ? TIPT_OK : fail_cuda(err, "ensemble class launch");
+        }
+    }
     RealStageParams p;
     memset(&p, 0, sizeof(p));
     p.phi = phi;
