@@ -79,3 +79,38 @@ def test_shared_chunks(storage):
             n, off = int(e.sizes[r]), int(e.offsets[r])
             for x, y in zip(out[0][2:], o[2:]):
                 assert torch.equal(x[..., off:off + n], y[..., off:off + n])
+
+
+@pytest.mark.parametrize("policy", [0, 2])
+def test_class_skips_and_reports_misaligned_replica(policy):
+    """A replica of a class whose offset is no multiple of 4 sites is left alone and reported,
+    whichever kernel the class takes; the others step."""
+    e = EN.Ensemble([EN.ReplicaSpec((8, 16, 64), 1.0, 0.05, seed=n) for n in range(3)],
+                    storage="f32c", check_every=2)
+    _, rids, act, n_act = e._march[0]
+    reps = (L.Replica * 3).from_buffer_copy(e._reps.cpu().numpy().tobytes())
+    reps[1].offset -= 1                     # inside the buffer
+    bad = torch.frombuffer(bytearray(bytes(reps)), dtype=torch.uint8).cuda()
+    out = []
+    try:
+        for table, entry in ((bad, "march"), (e._reps, "list")):
+            phi, pi = torch.full_like(e.phi[0], -7.0), torch.full_like(e.pi[0], -7.0)
+            args = (ptr(e.phi[0]), ptr(e.pi[0]), ptr(phi), ptr(pi), e.n_total, ptr(table))
+            L.set_kernel_policy(policy)
+            if entry == "march":
+                L.call("tipt_ensemble_step_march", *args, ptr(rids), 3, None, 8, 16, 64,
+                       ptr(e.active), e._sp, None, 0, stream_handle())
+                assert L.device_status(clear=True) == 3  # TIPT_ERR_ALIGN
+            else:
+                chunks = (L.Chunk * 3)(*[L.Chunk(r, 8192, 0) for r in range(3)])
+                dev = torch.frombuffer(bytearray(bytes(chunks)), dtype=torch.uint8).cuda()
+                L.call("tipt_ensemble_step", L.TIPT_F32C, *args, ptr(dev), 3, ptr(e.active),
+                       e._sp, None, 0, stream_handle())
+            torch.cuda.synchronize()
+            out.append((phi, pi))
+    finally:
+        L.set_kernel_policy(0)
+        L.device_status(clear=True)
+    for x, y in zip(*out):
+        assert torch.equal(x[:, :8192], y[:, :8192]) and torch.equal(x[:, 16384:], y[:, 16384:])
+        assert bool((x[:, 8192:16384] == -7.0).all())

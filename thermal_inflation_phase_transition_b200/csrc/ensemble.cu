@@ -43,6 +43,7 @@ struct EnsParams {
     const int32_t* n_rids;
     int cpr;
     uint32_t m1, m2;                     // tipt_replica's multipliers of the class
+    int* status;                         // tipt_device_status's word
     int pieces;                          // blocks that share a chunk
     const int32_t* active;
     double h1, h2, inv_dx2, eta, inv_mu2, inv_a2;
@@ -76,6 +77,10 @@ __global__ void __launch_bounds__(256) ensemble_stage_kernel(EnsParams e) {
         if (!e.active[ch.replica]) continue;
         tipt_replica rp = e.reps[ch.replica];
         if constexpr (CLASS) {
+            if (rp.offset & 3) {  // as the marching stage: skipped and reported
+                if (threadIdx.x == 0) atomicExch(e.status, (int)TIPT_ERR_ALIGN);
+                continue;
+            }
             const int64_t left = (int64_t)rp.n0 * rp.n1 * rp.n2 - ch.begin;
             ch.count = left < kClassChunk ? (int32_t)left : kClassChunk;
             rp.m1 = e.m1;
@@ -449,9 +454,11 @@ extern "C" int tipt_ensemble_step_march(const void* phi, const void* pi, void* p
             e.step = sp->noise_step;
             e.ctr = reinterpret_cast<const unsigned long long*>(counter);
             e.offset = offset;
+            cudaError_t err = device_status_word(&e.status);
+            if (err != cudaSuccess) return fail_cuda(err, "device status word");
             const int grid = stage_grid(e);
             ensemble_stage_kernel<TIPT_F32C, true><<<grid, 256, 0, (cudaStream_t)stream>>>(e);
-            cudaError_t err = cudaGetLastError();
+            err = cudaGetLastError();
             return err == cudaSuccess ? TIPT_OK : fail_cuda(err, "ensemble class launch");
         }
     }

@@ -1971,6 +1971,10 @@ int launch_complex_march(const ComplexStageParams& p, cudaStream_t st) {
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "complex marching kernel launch");
 }
 
+cudaError_t device_status_word(int** word) {
+    return cudaGetSymbolAddress(reinterpret_cast<void**>(word), g_device_status);
+}
+
 }  // namespace tipt
 
 using namespace tipt;

@@ -9,6 +9,9 @@ namespace tipt {
 bool march_supported(int storage, const RealStageParams& p, int* warps = nullptr);
 int launch_march(int storage, const RealStageParams& p, int64_t smem_table, cudaStream_t st);
 
+// Address of the current device's status word that tipt_device_status reads.
+cudaError_t device_status_word(int** word);
+
 // Batched ensemble: the replicas rids[0..n_rids) of one 3-D shape class on the
 // compensated-FP32 marching stage.
 bool ensemble_march_supported(int n0, int n1, int n2);
