@@ -317,9 +317,11 @@ int tipt_ensemble_step(int storage, const void* phi, const void* pi, void* phi_o
 
 /* The same step for the replicas rids[0..n_rids) of one 3-D shape class
  * (n0 x n1 x n2, n2 % 4 == 0, n0 >= 2), compensated-FP32 storage, on the
- * marching stage (shared-memory tiles fed by bulk copies); bitwise equal to
- * tipt_ensemble_step for those replicas.  The packed buffers (and n_total * 4
- * bytes) must be 16-byte aligned; the replicas' offsets multiples of 4 sites. */
+ * marching stage (shared-memory tiles fed by bulk copies) where that is the faster
+ * one, else on the work-list kernel; bitwise equal to tipt_ensemble_step for those
+ * replicas.  The packed buffers (and n_total * 4 bytes) must be 16-byte aligned; a
+ * replica whose offset is no multiple of 4 sites is skipped and reported by
+ * tipt_device_status. */
 int tipt_ensemble_march_supported(int32_t n0, int32_t n1, int32_t n2);  /* 1 or 0 */
 int tipt_ensemble_step_march(const void* phi, const void* pi, void* phi_out, void* pi_out,
                              int64_t n_total, const tipt_replica* replicas, const int32_t* rids,
