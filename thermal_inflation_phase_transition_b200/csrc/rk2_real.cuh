@@ -336,15 +336,17 @@ __device__ __forceinline__ float midpoint_f32(const P& p, float ph, float pv) {
 }
 // The same value, pi brought to FP64 by its bits: a float's sign, exponent and mantissa
 // fields as a double are the float times 2^-896, exactly, zeros and denormals included,
-// and h1s = h1 2^896 takes the factor.  For the kernels that the conversion unit bounds
-// (one warp instruction in eight cycles): the float32 script loops 313 -> 303 us (real,
-// 256^3) and 607 -> 583 us (complex, 512x512x64); the thermal stages lose 1 %.  (An
-// infinity becomes 2^128, which rounds to one again; a NaN is lost here, but phi's own
-// stencil carries it into every output.)
+// and h1s = h1 2^896 takes the factor.  An infinity or NaN needs the double's own largest
+// exponent field (left as it is, it would be 2^128 and more times h1, finite in float32).
+// For the kernels that the conversion unit bounds (one warp instruction in eight cycles):
+// the float32 script loops 313 -> 303 us (real, 256^3) and 607 -> 583 us (complex,
+// 512x512x64) when it came in, of which the exponent's two instructions are 1 % (290 ->
+// 293 us and 568 -> 574 us a step today); the thermal stages lose 1 %.
 template <class P>
 __device__ __forceinline__ float midpoint_f32_bits(const P& p, float ph, float pv) {
     const int b = __float_as_int(pv);
-    const double s = __hiloint2double((b >> 3) & (int)0x8FFFFFFF, b << 29);
+    const int hi = (b >> 3) & (int)0x8FFFFFFF;
+    const double s = __hiloint2double(fabsf(pv) < INFINITY ? hi : hi | 0x70000000, b << 29);
     return __double2float_rn(__fma_rn(p.h1s, s, (double)ph));
 }
 
