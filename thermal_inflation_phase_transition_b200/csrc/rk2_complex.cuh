@@ -89,11 +89,15 @@ template <bool TH = true>
 __device__ __forceinline__ void complex_force(const ComplexStageParams& p, const double* tab,
                                               double p1, double p2, double& d1, double& d2) {
     const double r2 = __fma_rn(p1, p1, __dmul_rn(p2, p2));
-    double inv, root;
-    rsqrt_sqrt<true>(r2 > 1e-60 ? r2 : 1e-60, inv, root);
-    // r2 beyond the reciprocal square root's range (|Phi| > 1e150, or NaN): NaN, as the
+    double inv, rho;
+    // r2 beyond the reciprocal square root's range (|Phi| > 1e150): NaN, as the
     // reference's inf / inf
-    const double rho = r2 > 1e-60 ? root : __dmul_rn(r2, inv);
+    rsqrt_sqrt<true>(r2, inv, rho);
+    if (!(r2 > 1e-60)) {   // the floor of the projection; V' is taken at rho itself
+        rsqrt_sqrt<true>(r2 * 0x1p400, inv, rho);
+        rho = r2 > 0.0 ? rho * 0x1p-200 : r2;   // 0 and NaN as they are
+        inv = 1e30;
+    }
     double dvdr;
     if (TH && p.vkind == TIPT_VP_THERMAL)
         // C:2605-2680 _vprime_complex_inline: V'(rho_safe) times phi_a * (1 / rho_safe)
