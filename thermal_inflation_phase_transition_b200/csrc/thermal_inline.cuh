@@ -65,11 +65,13 @@ inline ThermalSite thermal_site(const tipt_thermal& t, double T) {
     s.far_b = s.half_b / (s.T2 * 1e-20);
     s.far_f = s.half_f / (s.T2 * 1e-20);
     // x in (max(x_min, 1e-20), x_top) with room for rounding; none when T is not a
-    // normal positive number
+    // normal positive number, or when x_min < 0: the room, relative to x_top, may then be
+    // smaller than the rounding of x - x_min, and the segment has to be clamped
     const double lo = t.x_min > 1e-20 ? t.x_min : 1e-20, hi = s.xhi < s.xtop ? s.xhi : s.xtop;
     s.sq_lo = (lo * T) * (lo * T) * (1.0 + 1e-12);
     s.sq_hi = (hi * T) * (hi * T) * (1.0 - 1e-12);
-    if (!(s.sq_lo >= 1e-300 && s.sq_hi <= 1e300 && T > 0.0)) s.sq_lo = 1.0, s.sq_hi = 0.0;
+    if (!(s.sq_lo >= 1e-300 && s.sq_hi <= 1e300 && T > 0.0 && t.x_min >= 0.0))
+        s.sq_lo = 1.0, s.sq_hi = 0.0;
     return s;
 }
 
