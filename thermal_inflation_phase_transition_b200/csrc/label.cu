@@ -120,29 +120,38 @@ __device__ __forceinline__ uint32_t run_mask(uint32_t m, int q) {
     return (len < 32 ? (1u << len) - 1u : 0xffffffffu) << q;
 }
 
-// Labels of one tile of TI x TJ rows of TK sites: L[s] = linear index of the
-// smallest site of s's component within the tile (-1 where not masked).  Warps read
-// rows (8 passes of 32 / TK rows) into masks; then one thread per row walks its
-// runs, so that a warp works on 32 rows at once (a lane per site spent 2.5 times the
-// instructions: most lanes idle in every union); then warps write rows.
-template <int S, int TI, int TJ, int TK>
+// Labels of one tile of TI x TJ lattice rows of KS x TK sites: L[s] = linear index of
+// the smallest site of s's component within the tile (-1 where not masked).  A lattice
+// row is KS consecutive rows of TK sites here, joined where one ends and the next
+// begins.  Warps read rows (8 passes of 32 / TK rows) into masks; then one thread per
+// row walks its runs, so that a warp works on 32 rows at once (a lane per site spent 2.5
+// times the instructions: most lanes idle in every union); then warps write rows.
+template <int S, int TI, int TJ, int KS, int TK>
 __global__ void __launch_bounds__(256) label_tile_kernel(const void* f, double thr, float thrf,
                                                          int32_t* L, int n0, int n1, int n2) {
     constexpr int RPW = 32 / TK;  // rows per warp and pass
     constexpr int RS = TK + 1;    // entries per row, odd: rows in different banks
-    static_assert(TI * TJ * TK == 2048 && 32 % TK == 0, "eight warps of eight passes");
-    __shared__ int32_t s_l[TI * TJ * RS];  // union-find over the runs, at their first column
-    __shared__ uint32_t s_m[TI * TJ];      // mask of each row
-    const int ntk = (n2 + TK - 1) / TK, ntj = (n1 + TJ - 1) / TJ;
+    constexpr int ROWS = TI * TJ * KS, RI = TJ * KS;  // rows of a tile, and of a plane of it
+    static_assert(ROWS * TK == 2048 && 32 % TK == 0, "eight warps of eight passes");
+    __shared__ int32_t s_l[ROWS * RS];  // union-find over the runs, at their first column
+    __shared__ uint32_t s_m[ROWS];      // mask of each row
+    const int ntk = (n2 + KS * TK - 1) / (KS * TK), ntj = (n1 + TJ - 1) / TJ;
     const int tk = blockIdx.x % ntk, tr = blockIdx.x / ntk;
     const int ti = tr / ntj, tj = tr - ti * ntj;
     const int lane = threadIdx.x & 31, sub = lane / TK, c = lane % TK;
-    const int row0 = (threadIdx.x >> 5) * 8 * RPW + sub, k = tk * TK + c;
+    const int row0 = (threadIdx.x >> 5) * 8 * RPW + sub;
     const int64_t N = (int64_t)n0 * n1 * n2;
+    // the lattice site of column q of a tile's row
+    const auto place = [&](int row, int q, int& i, int& j, int& k) {
+        i = ti * TI + row / RI;
+        j = tj * TJ + row / KS % TJ;
+        k = (tk * KS + row % KS) * TK + q;
+    };
     bool on[8];
 #pragma unroll
     for (int it = 0; it < 8; ++it) {
-        const int row = row0 + it * RPW, i = ti * TI + row / TJ, j = tj * TJ + row % TJ;
+        int i, j, k;
+        place(row0 + it * RPW, c, i, j, k);
         on[it] = i < n0 && j < n1 && k < n2 && above<S>(f, (i * n1 + j) * n2 + k, N, thr, thrf);
     }
 #pragma unroll
@@ -153,10 +162,12 @@ __global__ void __launch_bounds__(256) label_tile_kernel(const void* f, double t
     }
     __syncthreads();
     const int row = threadIdx.x;
-    const bool walks = row < TI * TJ;
+    const bool walks = row < ROWS;
     const uint32_t m = walks ? s_m[row] : 0u;
-    const uint32_t mj = walks && row % TJ > 0 ? s_m[row - 1] : 0u;   // the row above (j - 1)
-    const uint32_t mi = walks && row >= TJ ? s_m[row - TJ] : 0u;     // the row behind (i - 1)
+    const uint32_t mj = walks && row % RI >= KS ? s_m[row - KS] : 0u;  // the row above (j - 1)
+    const uint32_t mi = walks && row >= RI ? s_m[row - RI] : 0u;       // the row behind (i - 1)
+    const uint32_t mk = KS > 1 && walks && row % KS > 0 ? s_m[row - 1] : 0u;  // the one before
+    const bool joined = KS > 1 && (m & 1u) && mk >> (TK - 1) & 1u;
     bool ok = true;
     // a run starts under the first run of the row above that it touches, or else of
     // the row behind: no union needed for that one
@@ -165,14 +176,15 @@ __global__ void __launch_bounds__(256) label_tile_kernel(const void* f, double t
         const uint32_t run = run_mask(rest, q);
         rest &= ~run;
         int parent = row * RS + q;
-        if (run & mj) parent = (row - 1) * RS + run_start(mj, __ffs((int)(run & mj)) - 1);
-        else if (run & mi) parent = (row - TJ) * RS + run_start(mi, __ffs((int)(run & mi)) - 1);
+        if (run & mj) parent = (row - KS) * RS + run_start(mj, __ffs((int)(run & mj)) - 1);
+        else if (run & mi) parent = (row - RI) * RS + run_start(mi, __ffs((int)(run & mi)) - 1);
+        else if (q == 0 && joined) parent = (row - 1) * RS + run_start(mk, TK - 1);
         s_l[row * RS + q] = parent;
     }
     __syncthreads();
     // the other overlaps unite; one with the row behind adds nothing where the rows
     // above both of them touch it in one column
-    const uint32_t both = mj && mi ? m & mj & mi & s_m[row - TJ - 1] : 0u;
+    const uint32_t both = mj && mi ? m & mj & mi & s_m[row - RI - KS] : 0u;
     for (uint32_t rest = m; rest;) {
         const int q = __ffs((int)rest) - 1;
         const uint32_t run = run_mask(rest, q);
@@ -182,7 +194,7 @@ __global__ void __launch_bounds__(256) label_tile_kernel(const void* f, double t
         for (; o;) {
             const int x = __ffs((int)o) - 1;
             o &= ~run_mask(o, x);
-            unite(s_l, row * RS + q, (row - 1) * RS + run_start(mj, x), ok);
+            unite(s_l, row * RS + q, (row - KS) * RS + run_start(mj, x), ok);
         }
         o = run & mi;
         if (o && !(run & mj)) o &= ~run_mask(o, __ffs((int)o) - 1);
@@ -190,8 +202,10 @@ __global__ void __launch_bounds__(256) label_tile_kernel(const void* f, double t
             const int x = __ffs((int)o) - 1;
             const uint32_t ov = run_mask(o, x);
             o &= ~ov;
-            if (!(ov & both)) unite(s_l, row * RS + q, (row - TJ) * RS + run_start(mi, x), ok);
+            if (!(ov & both)) unite(s_l, row * RS + q, (row - RI) * RS + run_start(mi, x), ok);
         }
+        if (q == 0 && joined && run & (mj | mi))
+            unite(s_l, row * RS, (row - 1) * RS + run_start(mk, TK - 1), ok);
     }
     __syncthreads();
     for (uint32_t rest = m; rest;) {
@@ -202,12 +216,16 @@ __global__ void __launch_bounds__(256) label_tile_kernel(const void* f, double t
     __syncthreads();
 #pragma unroll
     for (int it = 0; it < 8; ++it) {
-        const int row = row0 + it * RPW, i = ti * TI + row / TJ, j = tj * TJ + row % TJ;
+        const int row = row0 + it * RPW;
+        int i, j, k;
+        place(row, c, i, j, k);
         if (i >= n0 || j >= n1 || k >= n2) continue;
         int32_t l = -1;
         if (on[it]) {
-            const int r = s_l[row * RS + run_start(s_m[row], c)], rr = r / RS;
-            l = ((ti * TI + rr / TJ) * n1 + tj * TJ + rr % TJ) * n2 + tk * TK + r % RS;
+            const int r = s_l[row * RS + run_start(s_m[row], c)];
+            int ri, rj, rk;
+            place(r / RS, r % RS, ri, rj, rk);
+            l = (ri * n1 + rj) * n2 + rk;
         }
         L[(i * n1 + j) * n2 + k] = l;
     }
@@ -236,8 +254,7 @@ __global__ void __launch_bounds__(256) label_faces_kernel(int32_t* L, int n0, in
     const unsigned inner = (unsigned)(n1 * n2), nf = (unsigned)((n[d] - 1) / t[d]);
     const unsigned faces = nf + (periodic && n[d] > 1 ? 1u : 0u);
     const unsigned per = d == 0 ? inner : (unsigned)n[ou] * (unsigned)n[in];
-    // a direction with faces has two sites or more and tiles of eight or more: total <=
-    // N / 8 + N / 2 < 2^31, FastDiv's range (N < 2^31 sites)
+    // at most n[d] faces of N / n[d] sites: total <= N < 2^31, FastDiv's range
     const unsigned total = faces * per;
     const int lane = threadIdx.x & 31;
     bool ok = true;
@@ -414,34 +431,68 @@ static int grid_for(int64_t N) {
     return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
 
-// Tile labels, then the unions across tile faces.  Tiles: 8 x 8 rows of 32 sites,
-// 8 x 32 rows of 8 for short rows (fewer than 20 sites would leave lanes of the
-// 32-site rows idle), 64 rows of 32 of a single plane.
-template <int S, int TI, int TJ, int TK>
+// Tile labels, then the unions across tile faces.
+template <int S, int TI, int TJ, int KS, int TK>
 static void launch_tiles_as(const void* field, double thr, int32_t* L, int n0, int n1, int n2,
                             bool periodic, cudaStream_t st) {
     float thrf = (float)thr;
     if ((double)thrf > thr) thrf = nextafterf(thrf, -INFINITY);
-    const int64_t tiles = (int64_t)((n0 + TI - 1) / TI) * ((n1 + TJ - 1) / TJ) * ((n2 + TK - 1) / TK);
-    label_tile_kernel<S, TI, TJ, TK><<<(unsigned)tiles, 256, 0, st>>>(field, thr, thrf, L, n0, n1, n2);
+    constexpr int TR = KS * TK;  // sites of a tile along the rows
+    const int64_t tiles = (int64_t)((n0 + TI - 1) / TI) * ((n1 + TJ - 1) / TJ) * ((n2 + TR - 1) / TR);
+    label_tile_kernel<S, TI, TJ, KS, TK><<<(unsigned)tiles, 256, 0, st>>>(field, thr, thrf, L, n0, n1, n2);
     // the direction with the most face pairs sets the grid
     const int64_t N = (int64_t)n0 * n1 * n2;
     const int64_t pi = ((n0 - 1) / TI + 1) * (N / n0), pj = ((n1 - 1) / TJ + 1) * (N / n1),
-                  pk = ((n2 - 1) / TK + 1) * (N / n2);
+                  pk = ((n2 - 1) / TR + 1) * (N / n2);
     const int64_t most = pi > pj ? (pi > pk ? pi : pk) : (pj > pk ? pj : pk);
     const FaceDivs divs = {{FastDiv((uint32_t)(N / n0)), FastDiv((uint32_t)(N / n1)),
                             FastDiv((uint32_t)(N / n2))},
                            {FastDiv((uint32_t)n2), FastDiv((uint32_t)n2), FastDiv((uint32_t)n1)}};
-    label_faces_kernel<TI, TJ, TK><<<dim3((unsigned)grid_for(most), 3), 256, 0, st>>>(
+    label_faces_kernel<TI, TJ, TR><<<dim3((unsigned)grid_for(most), 3), 256, 0, st>>>(
         L, n0, n1, n2, divs, periodic ? 1 : 0);
 }
 
+// The tiles of a lattice: 8 x 8 rows of 32 sites, 8 x 32 rows of 8 for short rows (fewer
+// than 20 sites would leave lanes of the 32-site rows idle), 64 rows of 32 of a single
+// plane; a lattice that is thin in two directions, of which these would cover more than
+// four times its sites, takes the shape that covers it with the fewest tiles (an empty
+// tile costs 2.3 ns; float32 at a low threshold / above the field: 1 x 1 x 16e6 2836 /
+// 1184 -> 305 / 70 us, 8e6 x 1 x 2 5115 / 2820 -> 860 / 144, 2 x 2 x 4e6 1917 / 370 -> 613 /
+// 83, 1e6 x 4 x 4 1084 / 399 -> 320 / 101).
 template <int S>
 static void launch_tiles(const void* field, double thr, int32_t* L, int n0, int n1, int n2,
                          bool periodic, cudaStream_t st) {
-    if (n0 == 1) launch_tiles_as<S, 1, 64, 32>(field, thr, L, n0, n1, n2, periodic, st);
-    else if (n2 < 20) launch_tiles_as<S, 8, 32, 8>(field, thr, L, n0, n1, n2, periodic, st);
-    else launch_tiles_as<S, 8, 8, 32>(field, thr, L, n0, n1, n2, periodic, st);
+    using Launch = void (*)(const void*, double, int32_t*, int, int, int, bool, cudaStream_t);
+    struct Shape {
+        int ti, tj, tr;
+        Launch launch;
+    };
+    static const Shape longs[] = {{8, 8, 32, launch_tiles_as<S, 8, 8, 1, 32>},
+                                  {1, 64, 32, launch_tiles_as<S, 1, 64, 1, 32>},
+                                  {1, 1, 2048, launch_tiles_as<S, 1, 1, 64, 32>},
+                                  {1, 8, 256, launch_tiles_as<S, 1, 8, 8, 32>},
+                                  {8, 1, 256, launch_tiles_as<S, 8, 1, 8, 32>},
+                                  {2, 2, 512, launch_tiles_as<S, 2, 2, 16, 32>},
+                                  {64, 1, 32, launch_tiles_as<S, 64, 1, 1, 32>}};
+    static const Shape shorts[] = {{8, 32, 8, launch_tiles_as<S, 8, 32, 1, 8>},
+                                   {1, 256, 8, launch_tiles_as<S, 1, 256, 1, 8>},
+                                   {256, 1, 8, launch_tiles_as<S, 256, 1, 1, 8>},
+                                   {64, 4, 8, launch_tiles_as<S, 64, 4, 1, 8>},
+                                   {4, 64, 8, launch_tiles_as<S, 4, 64, 1, 8>}};
+    const bool single = n0 == 1, brief = !single && n2 < 20;
+    const auto tiles = [&](const Shape& t) {
+        return (int64_t)((n0 - 1) / t.ti + 1) * ((n1 - 1) / t.tj + 1) * ((n2 - 1) / t.tr + 1);
+    };
+    const Shape* pick = brief ? &shorts[0] : &longs[single ? 1 : 0];
+    if (tiles(*pick) * 512 > (int64_t)n0 * n1 * n2) {
+        const auto least = [&](const auto& shapes) {
+            for (const Shape& t : shapes)
+                if (tiles(t) < tiles(*pick)) pick = &t;
+        };
+        least(longs);
+        least(shorts);
+    }
+    pick->launch(field, thr, L, n0, n1, n2, periodic, st);
 }
 
 int64_t label_workspace_bytes(int64_t N) {
