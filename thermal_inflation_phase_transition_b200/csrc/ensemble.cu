@@ -58,8 +58,10 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t x, uint32_t m) { return m ? __
 
 constexpr int kClassChunk = 8192;
 
+// Bound by the latency of the loads: four blocks an SM (at three, with 76 registers, the
+// compensated kernel over a chunk list took 219 instead of 155 us for 1024 replicas of 128^2).
 template <int S, bool CLASS>
-__global__ void __launch_bounds__(256) ensemble_stage_kernel(EnsParams e) {
+__global__ void __launch_bounds__(256, S == TIPT_F32C ? 4 : 0) ensemble_stage_kernel(EnsParams e) {
     const uint64_t step = e.step + (e.ctr ? *e.ctr + (unsigned long long)e.offset : 0ull);
     // Blocks that share a chunk take its 256-thread passes in turn.
     const int stride = e.pieces * (int)blockDim.x;
@@ -313,13 +315,20 @@ __global__ void __cluster_dims__(kObsCta, 1, 1) __launch_bounds__(kObsThreads)
     }
 }
 
-// Few chunks are shared between blocks until eight blocks an SM have work: 128 chunks of
-// 8192 sites (64 replicas of 128^2) 33 us on one block each -> 16 us.
-static int stage_grid(EnsParams& e) {
-    const int resident = num_sms() * 8;
-    const int per = e.n_chunks < resident ? resident / e.n_chunks : 1;
-    e.pieces = per < 16 ? per : 16;
-    return e.n_chunks < resident ? e.n_chunks * e.pieces : resident;
+// Chunks are shared between blocks until an SM has sixteen blocks (four are resident, the others
+// even out the end), but not into less than a pass of the 256 threads each (chunk_sites: a
+// chunk's sites on average; two a thread in compensated FP32).  One block a chunk / this, in us:
+// 64 replicas of 128^2 17 / 14, 300 of 101 x 97 75 / 54, 1000 163 / 151, 1024 of 128^2 155 / 159,
+// one of 64^3 17 / 5.5; 200 of 8^3, cut into eleven 7.9, uncut 4.1.
+static int stage_grid(EnsParams& e, int storage, int64_t chunk_sites) {
+    const int most = num_sms() * 16;
+    const int64_t passes = chunk_sites / (storage == TIPT_F32C ? 512 : 256);
+    int64_t per = e.n_chunks < most ? (most + e.n_chunks - 1) / e.n_chunks : 1;
+    if (per > 16) per = 16;
+    if (per > passes) per = passes > 1 ? passes : 1;
+    e.pieces = (int)per;
+    const int64_t items = e.n_chunks * per;
+    return items < most ? (int)items : most;
 }
 
 // Whether the marching stage is the faster one for n_rids replicas of a class: a launch takes
@@ -369,7 +378,7 @@ extern "C" int tipt_ensemble_step(int storage, const void* phi, const void* pi, 
     e.offset = offset;
     e.rids = nullptr;
     e.n_rids = nullptr;
-    const int grid = stage_grid(e);
+    const int grid = stage_grid(e, storage, n_total / n_chunks);
     cudaStream_t st = (cudaStream_t)stream;
     if (storage == TIPT_F64) ensemble_stage_kernel<TIPT_F64, false><<<grid, 256, 0, st>>>(e);
     else ensemble_stage_kernel<TIPT_F32C, false><<<grid, 256, 0, st>>>(e);
@@ -456,7 +465,7 @@ extern "C" int tipt_ensemble_step_march(const void* phi, const void* pi, void* p
             e.offset = offset;
             cudaError_t err = device_status_word(&e.status);
             if (err != cudaSuccess) return fail_cuda(err, "device status word");
-            const int grid = stage_grid(e);
+            const int grid = stage_grid(e, TIPT_F32C, (int64_t)n0 * n1 * n2 / cpr);
             ensemble_stage_kernel<TIPT_F32C, true><<<grid, 256, 0, (cudaStream_t)stream>>>(e);
             err = cudaGetLastError();
             return err == cudaSuccess ? TIPT_OK : fail_cuda(err, "ensemble class launch");
