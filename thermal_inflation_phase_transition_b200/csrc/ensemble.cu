@@ -246,38 +246,51 @@ __global__ void __launch_bounds__(256, S == TIPT_F32C ? 4 : 0) ensemble_stage_ke
     }
 }
 
-// A cluster of kObsCta blocks per replica counts its sites with phi > thr (a whole number, so
-// the order is free) and adds the counts up in the first block's shared memory; 16-byte loads
+// The blocks of a replica (NC, a cluster) count its sites with phi > thr (a whole number, so
+// the order is free) and add the counts up in the first block's shared memory; 16-byte loads
 // where the replica's planes are aligned.  Bound by HBM: 112 replicas of 128^2, 64^3 and 96^3
-// (23.6 M sites) 970 us with one block of 256 threads a replica and single loads -> 58 us.
-constexpr int kObsCta = 8, kObsThreads = 512;
+// (23.6 M sites) 970 us with one block of 256 threads a replica and single loads -> 58 us on
+// clusters of eight blocks of 512 threads.
+struct ObsParams {
+    const void* phi;
+    int64_t n_total;
+    const tipt_replica* reps;
+    int32_t n_replicas;
+    int32_t* active;
+    int32_t* n_active;
+    double thr, stop_frac, retire_frac;
+    uint64_t step0;
+    const unsigned long long* ctr;
+    long long offset;
+    int64_t* first_step;
+    double* frac_out;
+};
 
-template <int S>
-__global__ void __cluster_dims__(kObsCta, 1, 1) __launch_bounds__(kObsThreads)
-    ensemble_observe_kernel(const void* phi, int64_t n_total, const tipt_replica* reps,
-                            int32_t n_replicas, int32_t* active, int32_t* n_active, double thr,
-                            double stop_frac, double retire_frac, uint64_t step0,
-                            const unsigned long long* ctr, long long offset, int64_t* first_step,
-                            double* frac_out) {
+template <int S, int NC, int NT>
+__device__ __forceinline__ void observe_replicas(const ObsParams& o) {
     namespace cg = cooperative_groups;
     using E = typename std::conditional<S == TIPT_F64, double, float>::type;
     using V = typename std::conditional<S == TIPT_F64, double2, float4>::type;
     constexpr int W = 16 / sizeof(E);
     __shared__ unsigned long long s_count;
     const cg::cluster_group cluster = cg::this_cluster();
-    const unsigned part = cluster.block_rank();
-    const uint64_t step = step0 + (ctr ? *ctr + (unsigned long long)offset : 0ull);
-    const int64_t t0 = (int64_t)part * kObsThreads + threadIdx.x;
-    constexpr int64_t kStride = (int64_t)kObsCta * kObsThreads;
-    for (int64_t r = blockIdx.x / kObsCta; r < n_replicas; r += gridDim.x / kObsCta) {
+    const unsigned part = NC > 1 ? cluster.block_rank() : 0;
+    const auto meet = [&] {
+        if constexpr (NC > 1) cluster.sync();
+        else __syncthreads();
+    };
+    const uint64_t step = o.step0 + (o.ctr ? *o.ctr + (unsigned long long)o.offset : 0ull);
+    const int64_t t0 = (int64_t)part * NT + threadIdx.x;
+    constexpr int64_t kStride = (int64_t)NC * NT;
+    for (int64_t r = blockIdx.x / NC; r < o.n_replicas; r += gridDim.x / NC) {
         if (threadIdx.x == 0) s_count = 0;
-        cluster.sync();
-        const tipt_replica rp = reps[r];
+        meet();
+        const tipt_replica rp = o.reps[r];
         const int64_t n = (int64_t)rp.n0 * rp.n1 * rp.n2;
-        const E* hi = static_cast<const E*>(phi) + rp.offset;
-        const E* lo = hi + n_total;  // float32 pairs
+        const E* hi = static_cast<const E*>(o.phi) + rp.offset;
+        const E* lo = hi + o.n_total;  // float32 pairs
         const auto above = [&](E a, E b) {
-            return (S == TIPT_F64 ? (double)a : (double)a + (double)b) > thr ? 1u : 0u;
+            return (S == TIPT_F64 ? (double)a : (double)a + (double)b) > o.thr ? 1u : 0u;
         };
         unsigned long long cnt = 0;
         const bool vec = reinterpret_cast<uintptr_t>(hi) % 16 == 0 &&
@@ -285,8 +298,20 @@ __global__ void __cluster_dims__(kObsCta, 1, 1) __launch_bounds__(kObsThreads)
         const int64_t nv = vec ? n / W : 0;
         const V* vh = reinterpret_cast<const V*>(hi);
         const V* vl = reinterpret_cast<const V*>(lo);
+        int64_t q = t0;
+        if constexpr (S == TIPT_F64) {
+            // eight loads in flight (unrolled by the compiler four times: 285 instead of 152 us
+            // for three replicas of 200x203x199, 8.4 instead of 4.5 us for 64 of 128^2)
+            for (; q + 7 * kStride < nv; q += 8 * kStride) {
+                V x[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) x[u] = __ldg(vh + q + u * kStride);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) cnt += above(x[u].x, 0.0) + above(x[u].y, 0.0);
+            }
+        }
 #pragma unroll 4
-        for (int64_t q = t0; q < nv; q += kStride) {
+        for (; q < nv; q += kStride) {
             const V x = __ldg(vh + q);
             if constexpr (S == TIPT_F64) {
                 cnt += above(x.x, 0.0) + above(x.y, 0.0);
@@ -295,24 +320,33 @@ __global__ void __cluster_dims__(kObsCta, 1, 1) __launch_bounds__(kObsThreads)
                 cnt += above(x.x, y.x) + above(x.y, y.y) + above(x.z, y.z) + above(x.w, y.w);
             }
         }
-        for (int64_t q = nv * W + t0; q < n; q += kStride)
+        for (q = nv * W + t0; q < n; q += kStride)
             cnt += above(__ldg(hi + q), S == TIPT_F64 ? E(0) : __ldg(lo + q));
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, m);
-        if ((threadIdx.x & 31) == 0) atomicAdd(cluster.map_shared_rank(&s_count, 0), cnt);
-        cluster.sync();
+        if ((threadIdx.x & 31) == 0)
+            atomicAdd(NC > 1 ? cluster.map_shared_rank(&s_count, 0) : &s_count, cnt);
+        meet();
         if (part == 0 && threadIdx.x == 0) {
             const double frac = (double)s_count / (double)n;
-            frac_out[r] = frac;
-            if (active[r]) {
-                if (frac > stop_frac && first_step[r] < 0) first_step[r] = (int64_t)step;
-                if (frac > retire_frac) {
-                    active[r] = 0;
-                    atomicSub(n_active, 1);
+            o.frac_out[r] = frac;
+            if (o.active[r]) {
+                if (frac > o.stop_frac && o.first_step[r] < 0) o.first_step[r] = (int64_t)step;
+                if (frac > o.retire_frac) {
+                    o.active[r] = 0;
+                    atomicSub(o.n_active, 1);
                 }
             }
         }
     }
+}
+template <int S>
+__global__ void __launch_bounds__(256) ensemble_observe_kernel(ObsParams o) {
+    observe_replicas<S, 1, 256>(o);
+}
+template <int S>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(512) ensemble_observe_cluster(ObsParams o) {
+    observe_replicas<S, 8, 512>(o);
 }
 
 // Chunks are shared between blocks until an SM has sixteen blocks (four are resident, the others
@@ -401,12 +435,19 @@ extern "C" int tipt_ensemble_observe(int storage, const void* phi, int64_t n_tot
         return fail(TIPT_ERR_ARG, "retire_frac must be >= stop_frac");
     if (n_replicas <= 0) return TIPT_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    const unsigned grid = (unsigned)(n_replicas < (1 << 24) ? n_replicas : 1 << 24) * kObsCta;
-    auto kern = storage == TIPT_F64 ? ensemble_observe_kernel<TIPT_F64>
-                                    : ensemble_observe_kernel<TIPT_F32C>;
-    kern<<<grid, kObsThreads, 0, st>>>(
-        phi, n_total, replicas, n_replicas, active, n_active, thr, stop_frac, retire_frac, step,
-        reinterpret_cast<const unsigned long long*>(counter), offset, first_step, frac_out);
+    // A cluster costs 80 ns of a full chip however little it counts, a single block 3 to 6 ns:
+    // single blocks for small replicas, and for middling ones (on average) where there are
+    // enough of them to fill the SMs.  Single / cluster in us, compensated FP32: 1024 of 128^2
+    // 28 / 80, 5000 of 16^2 14 / 275, 300 of 32^3 12 / 27, 400 of 40^3 37 / 58.
+    const int64_t sites = n_total / n_replicas;
+    const bool single = sites <= 16384 || (sites <= 65536 && n_replicas >= num_sms());
+    const ObsParams o{phi, n_total, replicas, n_replicas, active, n_active, thr, stop_frac,
+                      retire_frac, step, reinterpret_cast<const unsigned long long*>(counter), offset,
+                      first_step, frac_out};
+    const unsigned grid = (unsigned)(n_replicas < (1 << 24) ? n_replicas : 1 << 24);
+    const bool f64 = storage == TIPT_F64;
+    if (single) (f64 ? ensemble_observe_kernel<TIPT_F64> : ensemble_observe_kernel<TIPT_F32C>)<<<grid, 256, 0, st>>>(o);
+    else (f64 ? ensemble_observe_cluster<TIPT_F64> : ensemble_observe_cluster<TIPT_F32C>)<<<grid * 8, 512, 0, st>>>(o);
     cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? TIPT_OK : fail_cuda(err, "ensemble_observe launch");
 }
