@@ -52,21 +52,23 @@ __device__ __forceinline__ double force_d(const AltParams& p, double lap, double
     return __dsub_rn(__dmul_rn(p.inv_a2, lap), __dmul_rn(dv, p.inv_mu2));
 }
 
-// Any lattice shape on the column walk (column_walk.cuh); a table goes to shared memory once
-// per resident block.  Bound by the latency of the loads and of the force and noise chains.
-// Resident blocks per SM, measured at 3 / 4 / 5 / 6 (us): complex float32 256^3 overdamped
-// 239 / 245 / 255 / 257 (one site per thread with 64-bit divisions and seven reads: 281),
-// complex F32C 131x133x127 BAOAB 146 / 175 / 184 / 185 (193), complex FP64 192x190x188 BAOAB
-// 302 / 252 / 295 / 255 (289), real FP64 256^3 BAOAB 423 / 337 / 305 / 287 (417), real float32
-// 256^3 overdamped 169 / 166 / 165 / 166 (251).
-template <int S, bool CPLX>
+// Any lattice shape on the column walk (column_walk.cuh); V' tables are read in place.  Bound by
+// the latency of the loads and of the force and noise chains.  Resident blocks per SM, measured at
+// 3 / 4 / 5 / 6 (us): complex overdamped float32 256^3 245 / 250 / 263 / 263 (one site per thread
+// with 64-bit divisions and seven reads: 281), F32C 300x300x100 126 / 133 / 144 / 144, but FP64
+// 16x512x500 71 / 65 / 79 / 74; the complex BAOAB passes, which read pi as well, want four (both
+// passes at 3, then one of them at 3 / 4 / 5 / 6: F32C 2048x2000x1 pass 1 233 / 203 / 205 / 198,
+// pass 2 233 / 204 / 194 / 197, FP64 256^3 pass 1 681 / 626 / 647 / 626, pass 2 681 / 610 / 649 / 622);
+// real FP64 256^3 BAOAB 423 / 337 / 305 / 287 (417), real float32 256^3 overdamped 169 / 166 / 165 /
+// 166 (251).
+template <int S, bool CPLX, int MODE>
 constexpr int alt_blocks() {
-    return CPLX ? (S == TIPT_F64 ? 4 : 3) : 6;
+    return CPLX ? (S == TIPT_F64 || MODE != kOD ? 4 : 3) : 6;
 }
 
 // ----------------------------------------------------------------- real ----
 template <int S, int MODE, typename I>
-__global__ void __launch_bounds__(256, (alt_blocks<S, false>())) alt_real_kernel(AltParams p, ColumnGeom g) {
+__global__ void __launch_bounds__(256, (alt_blocks<S, false, MODE>())) alt_real_kernel(AltParams p, ColumnGeom g) {
     const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
     const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
     // the stored planes of a site: phi, or its hi and lo parts
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(256, (alt_blocks<S, false>())) alt_real_kernel
 
 // -------------------------------------------------------------- complex ----
 template <int S, int MODE, typename I>
-__global__ void __launch_bounds__(256, (alt_blocks<S, true>())) alt_complex_kernel(AltParams p, ColumnGeom g) {
+__global__ void __launch_bounds__(256, (alt_blocks<S, true, MODE>())) alt_complex_kernel(AltParams p, ColumnGeom g) {
     const bool zn = p.v.zn_active > 0.5 && p.v.zn_n > 0.5;
     const int64_t N = (int64_t)p.n0 * p.n1 * p.n2;
     const bool noisy = (MODE == kOD && p.ns != 0.0) || (MODE == kBA1 && p.c2 != 0.0);
@@ -260,7 +262,7 @@ static int launch_alt_k(const AltParams& p, cudaStream_t st) {
         kern = wide ? alt_real_kernel<S, MODE, int64_t> : alt_real_kernel<S, MODE, int>;
     unsigned blocks;
     const ColumnGeom g = column_geom(p.n0, p.n1, p.n2, 0, p.n0,
-                                     alt_blocks<S, CPLX>() * (int64_t)num_sms(), blocks);
+                                     alt_blocks<S, CPLX, MODE>() * (int64_t)num_sms(), blocks);
     kern<<<blocks, 256, 0, st>>>(p, g);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "integrator launch");
