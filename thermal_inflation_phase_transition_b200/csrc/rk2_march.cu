@@ -1579,22 +1579,34 @@ bool march_supported(int storage, const RealStageParams& p, int* warps) {
 }
 
 // How the work is split over `ctas` CTAs (MarchRuns), by the planes that the busiest
-// CTA computes: its items of CI planes, or an equal share of the (tile, plane) units.
-// Every run computes two planes' worth of prologue.  The equal shares put neighbouring
-// tiles at different planes, so a tile's halo rows are no longer in L2 from the
-// neighbour's reads: 6 % slower at 512^3 compensated FP32 with seven items a CTA (1.011
-// -> 1.075 ms), and that much they must save.  They matter below about 300^3, where
-// 64-plane items leave most SMs idle: 128^3 FP64 256 -> 36 us, 128^3 complex
-// compensated FP32 250 -> 53 us, 64^3 BAOAB 215 -> 32 us.
-static void split_work(MarchGeom& g, int tiles, int planes, int ctas, int loss) {
+// CTA computes: its items of CI planes (the last ones of a tile are shorter), or an equal
+// share of the (tile, plane) units.  Every run computes two planes' worth of prologue.
+// The equal shares put neighbouring tiles at different planes.  Where these lie further
+// apart than what L2 holds, a tile's halo rows are read twice (512^3 compensated FP32, 69
+// planes of 4 MB apart, seven items a CTA: 1.011 -> 1.075 ms), and the shares must save
+// `loss` percent; up to `near` bytes apart nothing (128x256x512, 35 MB: compensated FP32 147 ->
+// 134 us, FP64 245 -> 218, overdamped complex 165 -> 143).  The complex stage always loses
+// (near = 0; 128x128x512, 36 MB: 160 -> 178 us, although its shares are 9 % smaller).  The
+// shares matter below about 300^3, where 64-plane items leave most SMs idle: 128^3 FP64 256
+// -> 36 us, 128^3 complex compensated FP32 250 -> 53 us, 64^3 BAOAB 215 -> 32 us.
+static void split_work(MarchGeom& g, int tiles, int planes, int ctas, int loss, int64_t near) {
     const int64_t units = (int64_t)tiles * planes;
     const int64_t items = (int64_t)tiles * ((planes + g.CI - 1) / g.CI);
-    const int64_t rr = (items + ctas - 1) / ctas * ((g.CI < planes ? g.CI : planes) + 2);
-    const int64_t share = (units + ctas - 1) / ctas;
+    const auto rounds = [&](int64_t n) { return (n + ctas - 1) / ctas; };
+    const int64_t whole = (int64_t)tiles * (planes / g.CI);   // they come first
+    const int64_t rr = rounds(whole) * (g.CI + 2) + (rounds(items) - rounds(whole)) * (planes % g.CI + 2);
+    const int64_t share = rounds(units);
     const int64_t eq = share + 2 * (1 + (share + planes - 2) / planes);
+    // the next tile is `per` CTAs further on, `apart` planes from this one
+    const double exact = (double)units / ctas;
+    const int64_t per = exact < planes ? (int64_t)(planes / exact + 0.5) : 1;
+    const double apart = exact < planes ? (per * exact > planes ? per * exact - planes : planes - per * exact)
+                                        : (double)planes;
+    if (apart * tiles * g.stage_bytes <= (double)near) loss = 0;
     g.bal = eq * (100 + loss) < rr * 100 && units < 0x7FFFFFFF;
     g.items = (int)(g.bal ? units : items);
 }
+constexpr int64_t kHaloL2 = 64 << 20;   // half of L2
 
 // A batched ensemble's launch: its items run over the replicas.
 static bool has_replicas(const EnsMarch& em) { return em.reps != nullptr; }
@@ -1616,7 +1628,7 @@ static int launch_march_k(Kern kern, const RealStageParams& p, const MarchGeom& 
         return fail(TIPT_ERR_UNSUPPORTED, "marching kernel does not fit an SM (%d threads, %lld "
                     "bytes of shared memory)", threads, (long long)smem);
     int grid = num_sms() * per_sm;
-    if (!(has_replicas(extra) || ...)) split_work(g, g.nJB, p.i_end - p.i_begin, grid, 40 / g.TJ);
+    if (!(has_replicas(extra) || ...)) split_work(g, g.nJB, p.i_end - p.i_begin, grid, 40 / g.TJ, kHaloL2);
     if (grid > g.items) grid = g.items;
     kern<<<grid, threads, (size_t)smem, st>>>(p, g, extra...);
     e = cudaGetLastError();
@@ -1829,7 +1841,7 @@ static int launch_alt_march_k(const AltParams& p, cudaStream_t st) {
     if (e != cudaSuccess || per_sm < 1)
         return fail(TIPT_ERR_UNSUPPORTED, "integrator march kernel does not fit an SM");
     int grid = num_sms() * per_sm;
-    split_work(g, g.nJB, p.n0, grid, 40 / g.TJ);
+    split_work(g, g.nJB, p.n0, grid, 40 / g.TJ, kHaloL2);
     if (grid > g.items) grid = g.items;
     kern<<<grid, threads, (size_t)smem, st>>>(p, g);
     e = cudaGetLastError();
@@ -1948,7 +1960,7 @@ int launch_complex_march(const ComplexStageParams& p, cudaStream_t st) {
                        g.halo_off == 8 * 6 * 256 * 4 && g.stage_bytes == g.halo_off;
     const int threads = g.TJ * (g.KS / 2) + 32;
     int grid = num_sms() * ctas_per_sm(g, g.KS / 2);
-    split_work(g, g.nJB * g.nKS, p.n0, grid, 100 / g.TJ);
+    split_work(g, g.nJB * g.nKS, p.n0, grid, 100 / g.TJ, 0);
     if (grid > g.items) grid = g.items;
     const auto pick = [&](auto bal) {
         constexpr bool B = decltype(bal)::value;
