@@ -572,6 +572,12 @@ int tipt_device_status(int* status, int clear);
  * return; nothing is left in flight.  One launch only; position < 0 disarms. */
 int tipt_test_withhold_plane(int position);
 
+/* The same for the surrogate's tcgen05 kernels: in the next forward or gradient
+ * launch the waits of warp `warp` (1..7) of every block count as expired, once the
+ * product that they wait for has ended; the blocks report TIPT_ERR_TIMEOUT and
+ * return early.  One launch only; 0 disarms. */
+int tipt_test_expire_wait(int warp);
+
 #ifdef __cplusplus
 }
 #endif

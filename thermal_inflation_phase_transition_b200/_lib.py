@@ -142,6 +142,7 @@ _SIGS = {
     "tipt_set_march_fixed": [_i],
     "tipt_device_status": [C.POINTER(C.c_int), _i],
     "tipt_test_withhold_plane": [_i],
+    "tipt_test_expire_wait": [_i],
     "tipt_ensemble_march_supported": [C.c_int32, C.c_int32, C.c_int32],
     "tipt_ensemble_step_march": [_p, _p, _p, _p, _i64, _p, _p, C.c_int32, _p, C.c_int32,
                                  C.c_int32, C.c_int32, _p, C.POINTER(StepParams), _p, _i64, _p],
@@ -213,6 +214,12 @@ def test_withhold_plane(position: int) -> None:
     """Test of the bounded device waits: the next compensated-FP32 marching stage
     launch withholds ring position `position` in its block 0 (< 0 disarms)."""
     call("tipt_test_withhold_plane", int(position))
+
+
+def test_expire_wait(warp: int) -> None:
+    """Test of the bounded device waits: in the next tcgen05 launch of the surrogate the
+    waits of one warp (1..7; 0 disarms) of every block count as expired."""
+    call("tipt_test_expire_wait", int(warp))
 
 
 def device_status(clear: bool = False) -> int:

@@ -69,6 +69,7 @@ struct Args {
     int64_t rows_pad;
     float* partials;      // [tiles][kParams]
     float* loss_rows;     // [rows] or nullptr
+    int expire_warp;      // test: a warp of the tcgen05 kernels whose waits count as expired (0: none)
 };
 
 __device__ __forceinline__ uint32_t ld32(const bf16* p) {
@@ -528,6 +529,13 @@ __device__ __forceinline__ void load_x(const Args& a, int64_t row0, bf16* X) {
         st_chunk(X, rr, c0, R, f);
     }
 }
+// The block's wait for a product: false in every thread when the bounded wait of any of them
+// expired (the test's warp expires after the product has ended, so that nothing is in flight).
+__device__ __forceinline__ bool wait_product(const Args& a, uint64_t* bar, uint32_t phase) {
+    bool ok = mbar_wait(bar, phase);
+    if (a.expire_warp && (int)(threadIdx.x >> 5) == a.expire_warp) ok = false;
+    return __syncthreads_and(ok);
+}
 // TMEM columns (warp 0) and the barrier (thread 32); the caller's block barrier publishes both
 __device__ __forceinline__ void tc_begin(uint32_t* s_tmem, uint64_t* bar, uint32_t cols) {
     if (threadIdx.x < 32) {
@@ -598,9 +606,9 @@ __global__ void __launch_bounds__(kTcFwdThreads, 2) mlp_tc_forward_kernel(Args a
         }
         // the buffer of layer l - 1's weights is free: its product has ended
         if (l < 3) stage_w<NT>(a.params, l + 1, W + (~l & 1) * kTile);
-        ok = mbar_wait(bar, phase);
+        ok = wait_product(a, bar, phase);
         phase ^= 1u;
-        if (!__syncthreads_and(ok)) break;
+        if (!ok) break;
         tc_after();
         if (l < 3) {
 #pragma unroll 1
@@ -711,9 +719,9 @@ __global__ void __launch_bounds__(kGT, 1) mlp_tc_grad_kernel(Args a) {
         }
         if (l < 3) stage_w<kGT>(a.params, l + 1, l == 2 ? W3 : W1 + l * kTile);
         else transpose<kGT>(W3, WB, 32, 128);
-        ok = mbar_wait(bar, phase);
+        ok = wait_product(a, bar, phase);
         phase ^= 1u;
-        if (!__syncthreads_and(ok)) goto done;
+        if (!ok) goto done;
         tc_after();
         if (l < 3) {
             float z[16];
@@ -783,9 +791,9 @@ __global__ void __launch_bounds__(kGT, 1) mlp_tc_grad_kernel(Args a) {
             else gemm(tmem + kDw, DT, 128, Hl, l == 0 ? 16 : 128, kGR);  // dW^T[out][in]
             umma_commit(bar);
         }
-        ok = mbar_wait(bar, phase);
+        ok = wait_product(a, bar, phase);
         phase ^= 1u;
-        if (!__syncthreads_and(ok)) goto done;
+        if (!ok) goto done;
         tc_after();
         if (l > 0) {
             // dZ^T_{l-1} = dH^T * SiLU'(z_{l-1})
@@ -820,6 +828,7 @@ done:
 }
 
 int g_policy = 0;  // 0 automatic (tcgen05), 1 mma.sync, 2 tcgen05
+int g_expire_warp = 0;  // tipt_test_expire_wait: of the next launch
 
 int64_t tiles_of(int64_t rows) { return (rows + kRows - 1) / kRows; }
 
@@ -857,6 +866,14 @@ extern "C" int tipt_mlp_set_policy(int policy) {
     return TIPT_OK;
 }
 
+// Test of the bounded waits: in the next tcgen05 forward or gradient launch the waits of one warp
+// of every block count as expired.
+extern "C" int tipt_test_expire_wait(int warp) {
+    if (warp < 0 || warp > 7) return fail(TIPT_ERR_ARG, "warp must be in [0, 7] (0 disarms)");
+    g_expire_warp = warp;
+    return TIPT_OK;
+}
+
 extern "C" int64_t tipt_mlp_param_count(void) { return kParams; }
 
 extern "C" int64_t tipt_mlp_workspace_size(int64_t rows) {
@@ -881,6 +898,8 @@ extern "C" int tipt_mlp_forward(const float* params, const float* x, int64_t row
         if (e != cudaSuccess) return fail_cuda(e, "mlp forward attributes");
         mlp_kernel<false><<<(unsigned)tiles_of(rows), kThreads, kFwdSmem, (cudaStream_t)stream>>>(a);
     } else {
+        a.expire_warp = g_expire_warp;
+        g_expire_warp = 0;
         e = cudaFuncSetAttribute(mlp_tc_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kTcFwdSmem);
         if (e != cudaSuccess) return fail_cuda(e, "mlp forward attributes");
@@ -928,6 +947,8 @@ extern "C" int tipt_mlp_grad(const float* params, const float* x, const float* t
         static_assert(2 * kParams <= 3 * kRows * 128 + kParams, "gradient slices");
         tiles = (rows + kGR - 1) / kGR;
         a.partials = static_cast<float*>(workspace);
+        a.expire_warp = g_expire_warp;
+        g_expire_warp = 0;
         e = cudaFuncSetAttribute(mlp_tc_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kTcGradSmem);
         if (e != cudaSuccess) return fail_cuda(e, "mlp gradient attributes");
