@@ -543,7 +543,8 @@ int tipt_mlp_adam(float* params, const float* grad, float* m, float* v, const ui
 int tipt_set_kernel_policy(int policy);
 
 /* Marching-kernel tile shape: rows per tile, planes per work item and ring
- * stages (each 0 = automatic).  Performance only; used by the autotuner. */
+ * stages (each 0 = automatic).  While one is set, the calls that the marching
+ * kernels cover take them.  Performance only; used by the autotuner. */
 int tipt_set_march_tiles(int rows, int planes, int stages);
 
 /* Compensated-FP32 marching kernels compiled for a fixed geometry, used when the
@@ -555,7 +556,8 @@ int tipt_set_march_tiles(int rows, int planes, int stages);
 int tipt_set_march_fixed(int enable);
 
 /* Row segment of the complex marching kernel (sites per segment, a divisor of
- * nz of at least 128; 0 = automatic).  Performance only; used by the autotuner. */
+ * nz of at least 128; 0 = automatic); as a tile shape, it takes the calls that the
+ * kernel covers to it.  Performance only; used by the autotuner. */
 int tipt_set_march_kseg(int kseg);
 
 /* Device status word set by bounded device-side waits that expired

@@ -5,10 +5,12 @@ stages), plus the row segment for the complex kernel; ``field="real"`` tunes
 the real-field kernel, ``field="complex"`` the complex-field one (compensated
 FP32).  The built-in heuristic scores candidates by occupancy and halo share;
 ``tune`` instead times every admissible candidate on the device (CUDA events,
-inputs larger than L2 where the lattice is) and keeps the fastest.  Results are
+inputs larger than L2 where the lattice is) and keeps the fastest; ``default_ms`` is the
+call without one, whichever kernel the library takes for it.  Results are
 cached per (GPU name, field, storage, lattice shape, V' table size) in a JSON file
 (``$TIPT_AUTOTUNE_CACHE``, else ``~/.cache/tipt_b200/autotune.json``);
-``apply`` installs a cached shape, or the heuristic when there is none.
+``apply`` installs a cached shape that beats the default call, or the heuristic when
+there is none; a call that the marching kernels cover takes them while a shape is installed.
 
 No reference counterpart: the reference's only knob is the CPU tile size
 (R:1969-1970).
@@ -142,10 +144,12 @@ def tune(shape, storage="f32c", *, table_points=4096, steps=10, warmup=3, persis
     dev = torch.device(device)
     state = _state(shape, storage, dev, field)
     table = torch.linspace(-0.1, 0.1, table_points, dtype=torch.float64, device=dev)
-    L.set_kernel_policy(2)
     try:
         L.set_march_tiles(0, 0, 0)
+        L.set_march_kseg(0)
+        L.set_kernel_policy(0)
         default_ms = _time(state, table, steps, warmup, field)
+        L.set_kernel_policy(2)
         best, best_ms, tried = None, float("inf"), 0
         t_start = time.perf_counter()
         for c in candidates(shape, field):

@@ -277,7 +277,8 @@ static int launch_alt(int storage, const AltParams& p, cudaStream_t st) {
     // 240^3 260 / 285), and small lattices do not fill the pipeline (real BAOAB 32^3 14.8 /
     // 10.6, 64^3 13.1 / 16.0).
     const int64_t sites = (int64_t)p.n0 * p.n1 * p.n2;
-    const bool pays = p.n2 % 32 == 0 ? sites >= 1 << 18 : !CPLX && sites >= 12 << 20;
+    const bool pays = march_tiles_installed() ||
+                      (p.n2 % 32 == 0 ? sites >= 1 << 18 : !CPLX && sites >= 12 << 20);
     if (storage == TIPT_F32C && (kernel_policy() == 2 || (kernel_policy() == 0 && pays)) &&
         alt_march_supported(p, CPLX))
         return launch_alt_march(MODE, CPLX, p, st);

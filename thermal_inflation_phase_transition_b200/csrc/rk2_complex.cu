@@ -30,7 +30,8 @@ int launch_complex_stage(int storage, ComplexStageParams p, cudaStream_t st) {
     // 60, 256^3 290 / 580; 80^3 49 / 20, 112^3 75 / 43, 144^3 121 / 82, 208^3 247 / 233, 240^3
     // 322 / 347).
     const int64_t sites = (int64_t)p.n0 * p.n1 * p.n2;
-    const bool pays = sites >= (p.n2 % 32 == 0 ? 1 << 20 : 12 << 20);
+    const bool pays = march_tiles_installed() || march_kseg_installed() ||
+                      sites >= (p.n2 % 32 == 0 ? 1 << 20 : 12 << 20);
     if (storage == TIPT_F32C && (kernel_policy() == 2 || (kernel_policy() == 0 && pays))) {
         if (complex_march_supported(p)) return launch_complex_march(p, st);
         if (kernel_policy() == 2)

@@ -1588,7 +1588,7 @@ bool march_supported(int storage, const RealStageParams& p, int* warps) {
 // 134 us, FP64 245 -> 218, overdamped complex 165 -> 143).  The complex stage always loses
 // (near = 0; 128x128x512, 36 MB: 160 -> 178 us, although its shares are 9 % smaller).  The
 // shares matter below about 300^3, where 64-plane items leave most SMs idle: 128^3 FP64 256
-// -> 36 us, 128^3 complex compensated FP32 250 -> 53 us, 64^3 BAOAB 215 -> 32 us.
+// -> 36 us, 128^3 complex compensated FP32 250 -> 53 us, 64^3 BAOAB 215 -> 32 us.  Planes that were set (tipt_set_march_tiles) are kept.
 static void split_work(MarchGeom& g, int tiles, int planes, int ctas, int loss, int64_t near) {
     const int64_t units = (int64_t)tiles * planes;
     const int64_t items = (int64_t)tiles * ((planes + g.CI - 1) / g.CI);
@@ -1603,7 +1603,7 @@ static void split_work(MarchGeom& g, int tiles, int planes, int ctas, int loss, 
     const double apart = exact < planes ? (per * exact > planes ? per * exact - planes : planes - per * exact)
                                         : (double)planes;
     if (apart * tiles * g.stage_bytes <= (double)near) loss = 0;
-    g.bal = eq * (100 + loss) < rr * 100 && units < 0x7FFFFFFF;
+    g.bal = g_force_ci == 0 && eq * (100 + loss) < rr * 100 && units < 0x7FFFFFFF;
     g.items = (int)(g.bal ? units : items);
 }
 constexpr int64_t kHaloL2 = 64 << 20;   // half of L2
@@ -1982,6 +1982,9 @@ int launch_complex_march(const ComplexStageParams& p, cudaStream_t st) {
     e = cudaGetLastError();
     return e == cudaSuccess ? TIPT_OK : fail_cuda(e, "complex marching kernel launch");
 }
+
+bool march_tiles_installed() { return g_force_tj > 0 || g_force_ci > 0 || g_force_stages > 0; }
+bool march_kseg_installed() { return g_force_kseg > 0; }
 
 cudaError_t device_status_word(int** word) {
     return cudaGetSymbolAddress(reinterpret_cast<void**>(word), g_device_status);

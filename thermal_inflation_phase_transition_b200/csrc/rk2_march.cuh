@@ -9,6 +9,12 @@ namespace tipt {
 bool march_supported(int storage, const RealStageParams& p, int* warps = nullptr);
 int launch_march(int storage, const RealStageParams& p, int64_t smem_table, cudaStream_t st);
 
+// A tile shape (complex: or a row segment) is installed (tipt_set_march_tiles,
+// tipt_set_march_kseg): it was timed on the marching kernels, so the calls that these
+// cover take them, whatever the rule for the automatic shapes says.
+bool march_tiles_installed();
+bool march_kseg_installed();
+
 // Address of the current device's status word that tipt_device_status reads.
 cudaError_t device_status_word(int** word);
 

@@ -106,6 +106,7 @@ int launch_real_stage(int storage, RealStageParams p, cudaStream_t st) {
     int warps = 0;
     const bool march = g_kernel_policy == 2   ? march_supported(storage, p)
                        : g_kernel_policy == 1 ? false
+                       : march_tiles_installed() ? march_supported(storage, p)
                                               : march_pays(storage, p, sites, 16) &&
                                                     march_supported(storage, p, &warps) &&
                                                     march_pays(storage, p, sites, warps);
