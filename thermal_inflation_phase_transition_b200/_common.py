@@ -54,8 +54,12 @@ def ptr(t):
 def stream_handle(stream=None):
     if stream is not None:
         return C.c_void_p(stream.cuda_stream)
-    # the current stream's handle without a Stream object (0.6 us instead of 3.4)
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    # the current stream's handle without a Stream object (0.6 us instead of 3.4), where torch
+    # has the call (it is not part of its public interface)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(raw(torch.cuda.current_device()))
 
 
 def step_params(dt, dx, eta_eff, mu, inv_a2, noise_scale=0.0, noise_step=0, seed=0):
