@@ -454,11 +454,13 @@ static void launch_tiles_as(const void* field, double thr, int32_t* L, int n0, i
 
 // The tiles of a lattice: 8 x 8 rows of 32 sites, 8 x 32 rows of 8 for short rows (fewer
 // than 20 sites would leave lanes of the 32-site rows idle), 64 rows of 32 of a single
-// plane; a lattice that is thin in two directions, of which these would cover more than
-// four times its sites, takes the shape that covers it with the fewest tiles (an empty
-// tile costs 2.3 ns; float32 at a low threshold / above the field: 1 x 1 x 16e6 2836 /
-// 1184 -> 305 / 70 us, 8e6 x 1 x 2 5115 / 2820 -> 860 / 144, 2 x 2 x 4e6 1917 / 370 -> 613 /
-// 83, 1e6 x 4 x 4 1084 / 399 -> 320 / 101).
+// plane.  A lattice that is thin in two directions, of which these would cover more than
+// four times its sites with more tiles than are resident at once, takes the shape with
+// the fewest tiles and pairs across their faces, 360 pairs to a tile.  (A resident tile
+// costs nothing while it is empty: 2 x 2 x 5000 39 us in 157 tiles, 62 in ten; one that waits
+// costs 2.3 ns.)  Float32 at a low threshold / above the field: 1 x 1 x 16e6 2836 / 1184 -> 298 /
+// 69 us, 8e6 x 1 x 2 5115 / 2820 -> 804 / 143, 2 x 2 x 4e6 1917 / 370 -> 555 / 82, 1e6 x 4 x 4 1084 /
+// 399 -> 322 / 101.
 template <int S>
 static void launch_tiles(const void* field, double thr, int32_t* L, int n0, int n1, int n2,
                          bool periodic, cudaStream_t st) {
@@ -484,10 +486,15 @@ static void launch_tiles(const void* field, double thr, int32_t* L, int n0, int 
         return (int64_t)((n0 - 1) / t.ti + 1) * ((n1 - 1) / t.tj + 1) * ((n2 - 1) / t.tr + 1);
     };
     const Shape* pick = brief ? &shorts[0] : &longs[single ? 1 : 0];
-    if (tiles(*pick) * 512 > (int64_t)n0 * n1 * n2) {
+    if (tiles(*pick) * 512 > (int64_t)n0 * n1 * n2 && tiles(*pick) > 8 * (int64_t)num_sms()) {
+        const auto cost = [&](const Shape& t) {
+            const int64_t pairs = (n0 - 1) / t.ti * ((int64_t)n1 * n2) +
+                                  (n1 - 1) / t.tj * ((int64_t)n0 * n2) + (n2 - 1) / t.tr * ((int64_t)n0 * n1);
+            return 360 * tiles(t) + pairs;
+        };
         const auto least = [&](const auto& shapes) {
             for (const Shape& t : shapes)
-                if (tiles(t) < tiles(*pick)) pick = &t;
+                if (cost(t) < cost(*pick)) pick = &t;
         };
         least(longs);
         least(shorts);
