@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(256, (alt_blocks<S, true, MODE>())) alt_comple
 }
 
 // ------------------------------------------------------------------ host ----
+// Longest V' row that the marching kernels stage; longer ones take FP64 lookups in place.
 constexpr int64_t kMaxAltTableSmem = 96 * 1024;
 
 template <int S, int MODE, bool CPLX>
@@ -273,9 +274,10 @@ static int launch_alt(int storage, const AltParams& p, cudaStream_t st) {
     // compensated FP32 on the marching ring where the shape allows and it pays (bitwise the
     // generic kernel's results; kernel_policy 1 forces the generic one).  Rows that are not
     // whole 128-byte lines are copied one by one (march / generic in us, complex overdamped
-    // 80^3 31 / 13, 112^3 68 / 25, 240^3 239 / 191; real BAOAB 80^3 38 / 22, 208^3 204 / 191,
-    // 240^3 260 / 285), and small lattices do not fill the pipeline (real BAOAB 32^3 14.8 /
-    // 10.6, 64^3 13.1 / 16.0).
+    // 80^3 31 / 10, 112^3 68 / 22, 208^3 184 / 126, 240^3 237 / 193, 700x240x240 646 / 544; complex
+    // BAOAB 112^3 137 / 51, 208^3 372 / 362, but 240^3 477 / 537; real BAOAB 80^3 38 / 22, 208^3
+    // 204 / 191, 240^3 260 / 285) and have no tile above 256 sites; small lattices do not fill
+    // the pipeline (real BAOAB 32^3 14.8 / 10.6, 64^3 13.1 / 9.8).
     const int64_t sites = (int64_t)p.n0 * p.n1 * p.n2;
     const bool pays = march_tiles_installed() ||
                       (p.n2 % 32 == 0 ? sites >= 1 << 18 : !CPLX && sites >= 12 << 20);

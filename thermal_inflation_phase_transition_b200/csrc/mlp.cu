@@ -5,15 +5,15 @@
 // (zero-padded to 32), SiLU after the hidden layers.  Parameters are one FP32
 // vector, per layer W[in][out] then b[out]; every kernel converts the weights
 // it needs to BF16 in shared memory.  Matrix products take BF16 operands and
-// accumulate in FP32 (mma.sync m16n8k16).
+// accumulate in FP32: tcgen05.mma by default, mma.sync m16n8k16 by policy.
 //
-// One CTA owns a tile of 128 rows (8 warps x 16 rows) and carries it through
-// every layer without leaving the SM: activations stay in shared memory, only
-// the FP32 pre-activations of the hidden layers go to a global scratch for the
-// backward pass of the same CTA.  The gradient kernel fuses forward, loss and
-// backward; its per-tile parameter gradients go to a per-CTA slice of the
-// workspace and a second kernel sums the slices in a fixed order, so training
-// is deterministic.
+// One CTA owns a tile of rows (128; 64 in the tcgen05 gradient) and carries it
+// through every layer without leaving the SM: activations stay in shared memory,
+// the FP32 pre-activations of the hidden layers in tensor memory (mma.sync: in a
+// global scratch) for the backward pass of the same CTA.  The gradient kernels fuse
+// forward, loss and backward; their per-tile parameter gradients go to a per-CTA
+// slice of the workspace and a second kernel sums the slices in a fixed order, so
+// training is deterministic.
 //
 // Loss per row (targets row: event, exposure, w_gamma, w_curve, f_1..f_16):
 //   w_gamma (exp(l) exposure - event l) + w_curve/16 sum_k (softplus(o_k) - f_k o_k)
@@ -365,10 +365,11 @@ __global__ void mlp_adam_kernel(float* p, const float* g, float* m, float* v,
 // (the M or N extent) is stored as K/8 column chunks, each holding the R rows'
 // 8 consecutive K values (16 bytes) back to back, so an 8 x 8 core matrix is 128
 // contiguous bytes; descriptor LBO (next chunk along K) = 16 R bytes and SBO
-// (next 8-row group) = 128 bytes.  Accumulators live in tensor memory: lane =
-// tile row, column = output feature; one thread issues the MMAs and commits
-// them to an mbarrier that every thread waits on with a time limit.  Warps w
-// and w + 4 read the same 32 TMEM lanes (w % 4) and split the columns.
+// (next 8-row group) = 128 bytes.  Accumulators live in tensor memory (forward:
+// lane = tile row, column = output feature; gradient: lane = feature, column = row);
+// one thread issues the MMAs and commits them to an mbarrier that every thread waits
+// on with a time limit.  Warps w, w + 4, ... read the same 32 TMEM lanes (w % 4) and
+// split the columns.
 
 __device__ int g_mlp_status = 0;  // TIPT_ERR_TIMEOUT after a bounded wait expired
 constexpr uint64_t kWaitNs = 2000000000ull;

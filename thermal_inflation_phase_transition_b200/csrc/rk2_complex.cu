@@ -11,6 +11,7 @@
 
 namespace tipt {
 
+// Longest V' row that the marching kernel stages; longer ones take FP64 lookups.
 constexpr int64_t kMaxTableSmemC = 96 * 1024;
 
 template <int S>

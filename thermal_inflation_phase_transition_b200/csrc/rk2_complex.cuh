@@ -34,7 +34,7 @@ struct ComplexStageParams {
     const double* table;
     double tmin, dinv;
     double c1, c2, c3;
-    int table_in_smem;
+    int table_in_smem;  // as RealStageParams::table_in_smem
     ThermalSite th;  // TIPT_VP_THERMAL: the inline thermal V'(rho) at T
     // Range of the new |Phi| (optional, the complex loop's per-step rho check,
     // C:4263-4288): as RealStageParams::range, folded from rho = sqrt(phi1^2 +

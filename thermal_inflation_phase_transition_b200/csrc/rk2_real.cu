@@ -77,7 +77,8 @@ static void canonical_shape(RealStageParams& p) {
 //    / 508, with 12 and more 224^3 173 / 191, 256^3 223 / 259, 384^3 836 / 890;
 //  * compensated FP32 halves the instructions of the generic kernel where rows are whole
 //    128-byte lines (128^3 25.6 / 36.6, 256^3 134 / 254); other rows are copied one by one
-//    (80^3 48 / 12, 112^3 68 / 25, 208^3 178 / 151, 240^3 228 / 225);
+//    (80^3 48 / 12, 112^3 68 / 25, 208^3 178 / 140, 240^3 228 / 210) and have no tile above 256
+//    sites (the consumers of such a row's tile would be more than 512);
 //  * inline thermal V', long FP64 chains: 256^3, two halves, FP64 1032 / 841, float32 1009 /
 //    894; compensated FP32, whose stencil reads four components, 256^3 804 / 853, 96^3 67 / 54;
 //  * a noise array in the FP64 and float32 storages, loaded where the hash would be drawn (the

@@ -35,7 +35,10 @@ struct RealStageParams {
     int nT;
     double T_min, T_dinv, T;
     double c1, c2, c3;
-    int table_in_smem;   // 1: stage (and blend) the row into dynamic smem
+    // 1: the V' row is short enough for shared memory, where the marching kernels stage (and
+    // blend) it; the generic kernel reads it in place either way, in compensated FP32 with
+    // FP32 lookups as from the staged row (0: FP64 lookups in the global table)
+    int table_in_smem;
     // Device-resident schedule (for graph-captured step loops): when sched is
     // set, the step is s = *ctr + offset, row e = min(s, sched_len - 1) of
     // sched_cols doubles gives T = sched[cols e], the noise amplitude

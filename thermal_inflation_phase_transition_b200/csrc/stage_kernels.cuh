@@ -15,8 +15,8 @@ inline int stage_begin(const ComplexStageParams&) { return 0; }
 inline int stage_end(const ComplexStageParams& p) { return p.n0; }
 
 // Walks columns (column_walk.cuh); float32 storage keeps the midpoint values along the
-// column too, five conversions and back a site instead of seven.  The resident blocks
-// stage a table row once each.
+// column too, five conversions and back a site instead of seven.  V' rows are read in
+// place through L1, a 2-D table's two rows blended at each lookup.
 //
 // Bound: the latency of the loads and of the FP64 chains (64 registers a thread, four
 // blocks an SM; five or six blocks spill), then issue and, in float32 storage, the

@@ -211,7 +211,7 @@ struct ComplexSite {
         } else {
             // FP64 arithmetic after the neighbour sums.  The Laplacian of phi~ = phi + h1 pi
             // is lap + h1 lap(pi); float32 storage takes it from the float32 phi~ and rounds
-            // the midpoint's pi, as the reference stores them (see update_f32).
+            // the midpoint's pi, as the reference stores them (see update_f32_mid).
             const auto lap_of = [&](const E v[7], double c) {
                 const E s6 = v[1] + v[2] + v[3] + v[4] + v[5] + v[6];
                 return __dmul_rn(__fma_rn(-6.0, c, (double)s6), p.inv_dx2);
