@@ -277,7 +277,8 @@ static int launch_alt(int storage, const AltParams& p, cudaStream_t st) {
     // 80^3 31 / 10, 112^3 68 / 22, 208^3 184 / 126, 240^3 237 / 193, 700x240x240 646 / 544; complex
     // BAOAB 112^3 137 / 51, 208^3 372 / 362, but 240^3 477 / 537; real BAOAB 80^3 38 / 22, 208^3
     // 204 / 191, 240^3 260 / 285) and have no tile above 256 sites; small lattices do not fill
-    // the pipeline (real BAOAB 32^3 14.8 / 10.6, 64^3 13.1 / 9.8).
+    // the pipeline (real BAOAB 32^3 14.8 / 10.6; 64^3 13.1 / 16.0 when the generic kernel staged
+    // its table, 13.1 / 9.8 since it reads it in place: the line could lie higher).
     const int64_t sites = (int64_t)p.n0 * p.n1 * p.n2;
     const bool pays = march_tiles_installed() ||
                       (p.n2 % 32 == 0 ? sites >= 1 << 18 : !CPLX && sites >= 12 << 20);
