@@ -532,10 +532,12 @@ __device__ __forceinline__ void load_x(const Args& a, int64_t row0, bf16* X) {
 }
 // The block's wait for a product: false in every thread when the bounded wait of any of them
 // expired (the test's warp expires after the product has ended, so that nothing is in flight).
-__device__ __forceinline__ bool wait_product(const Args& a, uint64_t* bar, uint32_t phase) {
-    bool ok = mbar_wait(bar, phase);
-    if (a.expire_warp && (int)(threadIdx.x >> 5) == a.expire_warp) ok = false;
-    return __syncthreads_and(ok);
+__device__ __forceinline__ bool wait_product(bool patient, uint64_t* bar, uint32_t phase) {
+    const bool ended = mbar_wait(bar, phase);
+    return __syncthreads_and(ended && patient);
+}
+__device__ __forceinline__ bool patient_warp(const Args& a) {
+    return a.expire_warp == 0 || (int)(threadIdx.x >> 5) != a.expire_warp;
 }
 // TMEM columns (warp 0) and the barrier (thread 32); the caller's block barrier publishes both
 __device__ __forceinline__ void tc_begin(uint32_t* s_tmem, uint64_t* bar, uint32_t cols) {
@@ -598,6 +600,7 @@ __global__ void __launch_bounds__(kTcFwdThreads, 2) mlp_tc_forward_kernel(Args a
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);  // this warp's lane quarter
     uint32_t phase = 0;
     bool ok = true;
+    const bool patient = patient_warp(a);
 #pragma unroll 1
     for (int l = 0; l < 4; ++l) {
         if (tid == 0) {
@@ -607,7 +610,7 @@ __global__ void __launch_bounds__(kTcFwdThreads, 2) mlp_tc_forward_kernel(Args a
         }
         // the buffer of layer l - 1's weights is free: its product has ended
         if (l < 3) stage_w<NT>(a.params, l + 1, W + (~l & 1) * kTile);
-        ok = wait_product(a, bar, phase);
+        ok = wait_product(patient, bar, phase);
         phase ^= 1u;
         if (!ok) break;
         tc_after();
@@ -699,6 +702,7 @@ __global__ void __launch_bounds__(kGT, 1) mlp_tc_grad_kernel(Args a) {
     const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);  // this warp's lane quarter
     uint32_t phase = 0;
     bool ok = true;
+    const bool patient = patient_warp(a);
     float* part = a.partials + (int64_t)blockIdx.x * kParams;
     // sums of the tile's rows by the lane quarter of rows, then over the quarters
     const auto put_dz = [&](float (&g)[16], int N) {
@@ -720,7 +724,7 @@ __global__ void __launch_bounds__(kGT, 1) mlp_tc_grad_kernel(Args a) {
         }
         if (l < 3) stage_w<kGT>(a.params, l + 1, l == 2 ? W3 : W1 + l * kTile);
         else transpose<kGT>(W3, WB, 32, 128);
-        ok = wait_product(a, bar, phase);
+        ok = wait_product(patient, bar, phase);
         phase ^= 1u;
         if (!ok) goto done;
         tc_after();
@@ -792,7 +796,7 @@ __global__ void __launch_bounds__(kGT, 1) mlp_tc_grad_kernel(Args a) {
             else gemm(tmem + kDw, DT, 128, Hl, l == 0 ? 16 : 128, kGR);  // dW^T[out][in]
             umma_commit(bar);
         }
-        ok = wait_product(a, bar, phase);
+        ok = wait_product(patient, bar, phase);
         phase ^= 1u;
         if (!ok) goto done;
         tc_after();
